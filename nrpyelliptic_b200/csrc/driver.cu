@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "driver.cuh"
+#include "resident.cuh"
 
 namespace nrpyell {
 
@@ -324,6 +325,25 @@ RelaxResult relax_loop(const Dims& d, RfmTables* rt, BcTables* bt, L2Tables* lt,
 template RelaxResult relax_loop<double>(const Dims&, RfmTables*, BcTables*, L2Tables*, FusedWork*, Scratch*, int,
                                         const StateBuffers&, const RelaxParams&);
 template RelaxResult relax_loop<float>(const Dims&, RfmTables*, BcTables*, L2Tables*, FusedWork*, Scratch*, int,
+                                       const StateBuffers&, const RelaxParams&);
+
+template <typename T>
+RelaxResult relax_grid(const Dims& d, RfmTables* rt, BcTables* bt, L2Tables* lt, FusedWork* w, Scratch* s,
+                       const StateBuffers& b, const RelaxParams& rp) {
+  if constexpr (sizeof(T) == 8) {
+    if (resident_ok<T>(d)) {
+      std::vector<RelaxResult> r;
+      const ResGrid g = {d, rt, bt, lt, b, rp, w->state, (rp.history_buf ? rp.history_buf : w->history) + rp.history_offset};
+      if (!relax_resident<T>({g}, &r)) return {0, false, NAN};
+      return r[0];
+    }
+  }
+  const int tile = tuned_tile<T>(d, rt, bt, w, s, b, rp, lt);
+  return relax_loop<T>(d, rt, bt, lt, w, s, tile, b, rp);
+}
+template RelaxResult relax_grid<double>(const Dims&, RfmTables*, BcTables*, L2Tables*, FusedWork*, Scratch*,
+                                        const StateBuffers&, const RelaxParams&);
+template RelaxResult relax_grid<float>(const Dims&, RfmTables*, BcTables*, L2Tables*, FusedWork*, Scratch*,
                                        const StateBuffers&, const RelaxParams&);
 
 __global__ void k_correction_base(Dims d, const double* __restrict__ U, const double* __restrict__ aux,

@@ -73,6 +73,11 @@ int tuned_tile(const Dims& d, RfmTables* rt, BcTables* bt, FusedWork* w, Scratch
 template <typename T>
 RelaxResult relax_loop(const Dims& d, RfmTables* rt, BcTables* bt, L2Tables* lt, FusedWork* w, Scratch* s, int tile,
                        const StateBuffers& b, const RelaxParams& rp);
+// One grid's relaxation from b.y: on chip (kernels_resident.cu) where the
+// grid fits and no tile shape is forced, else relax_loop with the tuned shape.
+template <typename T>
+RelaxResult relax_grid(const Dims& d, RfmTables* rt, BcTables* bt, L2Tables* lt, FusedWork* w, Scratch* s,
+                       const StateBuffers& b, const RelaxParams& rp);
 // Correction form of the mixed-precision driver (nrpyell_relax_mixed): from
 // the FP64 base state U, its RHS rhs (interior and radiation ghost points)
 // and its residual bracket res (interior), the FP32 inputs of the correction

@@ -14,6 +14,9 @@ namespace nrpyell {
 
 // Upwind first-derivative weights (one copy per translation unit).
 static __constant__ double c_fd1w[11][11] = NRPYELL_FD1_UPWIND_INIT;
+// The same as literals, where the index is known at compile time: constant
+// memory loads hoisted out of a time loop took 132 registers.
+static __device__ const double kFd1w[11][11] = NRPYELL_FD1_UPWIND_INIT;
 
 template <typename T>
 struct SubDev {
@@ -293,10 +296,10 @@ __device__ __forceinline__ double radiation_sum_x0(const double* w, const double
   return d;
 }
 __device__ __forceinline__ double radiation_sum_x1(const double* v) {
-  double d = c_fd1w[5][0] * v[0];
+  double d = kFd1w[5][0] * v[0];
 #pragma unroll
   for (int m = 1; m < 11; m++)
-    if (m != 5) d = d + c_fd1w[5][m] * v[m];
+    if (m != 5) d = d + kFd1w[5][m] * v[m];
   return d;
 }
 
@@ -306,6 +309,23 @@ __device__ __forceinline__ double radiation_drf(double d0, double d1, double inv
   d0 *= invdx0;
   d1 *= invdx1;
   return dx0dr * d0 + dx1dr * d1;
+}
+
+// One outer layer of the radiation BC (apply_bcs_outerradiation_and_inner.c:
+// 400-407): the outgoing wave's d f/d r + f / r at the interior neighbour (X,
+// radius rn, cubed rn3) and at the point (Y, 1 / radius rinv), and the point's RHS from
+// the neighbour's, kprev.  The roundings are spelled out, so that the column
+// blocks and the on-chip radiation blocks agree bit for bit.
+__device__ __forceinline__ double radiation_outgoing_neighbour(double drf, double f, double rn) {
+  return __dadd_rn(drf, __ddiv_rn(f, rn));
+}
+__device__ __forceinline__ double radiation_outgoing_point(double drf, double f, double rinv) {
+  return __fma_rn(f, rinv, drf);
+}
+__device__ __forceinline__ double radiation_r3(double r) { return __dmul_rn(__dmul_rn(r, r), r); }
+__device__ __forceinline__ double radiation_layer(double cw, double kprev, double X, double Y, double rn3, double rinv) {
+  const double K = __dmul_rn(rn3, __fma_rn(cw, X, kprev));
+  return __fma_rn(__dmul_rn(__dmul_rn(K, rinv), rinv), rinv, __dmul_rn(-cw, Y));
 }
 
 // RHS of one gridfunction on the five outer layers of a column, inner to
@@ -318,14 +338,10 @@ __device__ __forceinline__ void radiation_layers(double cw, double kprev, const 
 #pragma unroll
   for (int L = 0; L < NGHOSTS; L++) {
     const double rn = __ldg(rcol + L * N1);
-    const double rr = __ldg(rcol + (L + 1) * N1);
-    const double out_int = -cw * (drf[L] + fvs[L] / rn);
-    const double K = rn * rn * rn * (kprev - out_int);
-    const double rinv = 1.0 / rr;
-    const double outw = -cw * (drf[L + 1] + fvs[L + 1] * rinv);
-    const double k = outw + K * rinv * rinv * rinv;
-    kk[L] = k;
-    kprev = k;
+    const double rinv = 1.0 / __ldg(rcol + (L + 1) * N1);
+    kprev = radiation_layer(cw, kprev, radiation_outgoing_neighbour(drf[L], fvs[L], rn),
+                            radiation_outgoing_point(drf[L + 1], fvs[L + 1], rinv), radiation_r3(rn), rinv);
+    kk[L] = kprev;
   }
 }
 
