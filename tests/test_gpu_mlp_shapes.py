@@ -55,3 +55,18 @@ def test_products(lib, n_in, width, depth, n_out, rows):
     for d in (full, dx, dt, dy):
         d.free()
     lib.nrpyell_mlp_destroy(m)
+
+
+@pytest.mark.parametrize("ntot", [1, 2, 511, 512, 4097])
+@pytest.mark.parametrize("K", [1, 15, 16, 17, 300])
+def test_pod_reconstruction(lib, ntot, K):
+    rng = np.random.default_rng(K)
+    mean, basis, c = (rng.normal(size=s).astype(np.float32) for s in ((ntot,), (K, ntot), (K,)))
+    dm, db, dc, dy = Dev(lib, mean), Dev(lib, basis), Dev(lib, c), Dev(lib, np.zeros(4 * ntot))
+    assert lib.nrpyell_pod_guess(dm.p, db.p, K, ntot, dc.p, 7.0, dy.p) == 0
+    y = dy.get((4 * ntot,)).view(np.float64).reshape(2, ntot)
+    ref = mean.astype(np.float64) + c.astype(np.float64) @ basis.astype(np.float64)
+    np.testing.assert_allclose(y[0], ref, rtol=0, atol=1e-13 * (1 + np.max(np.abs(ref))))
+    np.testing.assert_array_equal(y[1], 7.0 * y[0])
+    for d in (dm, db, dc, dy):
+        d.free()
