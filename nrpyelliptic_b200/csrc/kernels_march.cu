@@ -68,6 +68,12 @@ struct MarchSmem {
   static constexpr size_t bytes = march > cols ? march : cols;
 };
 
+// Whether a substep sweeps its planes (and, in a batch, its grids) from the
+// last to the first.  A substep touches 11 fields, more than L2 holds from
+// 256x256x32 on, and blocks run in index order, so sweeping every substep the
+// same way evicts each plane before the next substep comes to it.
+__device__ constexpr bool march_reversed(int stage) { return stage == 2 || stage == 4; }
+
 // Block `bid` of one grid's marching launch; dsm is the block's dynamic
 // shared memory (MarchSmem::bytes).  The radiation column blocks come after
 // the interior blocks (COLS_LAST: their short, latency-bound blocks fill the
@@ -90,12 +96,15 @@ __device__ __forceinline__ void march_block(const SubDev<T>& a, const int bid, d
   const int C = a.tiles0 * a.tiles1, nbig = C * a.mbig;
   const int s = b - nbig;
   const int col = b < nbig ? b % C : s % C;
-  const int z0 = NGHOSTS + (b < nbig ? (b / C) * PZ : a.mbig * PZ + (s / C) * a.msmall);
+  const int zf = b < nbig ? (b / C) * PZ : a.mbig * PZ + (s / C) * a.msmall;
   const int zc = b < nbig ? PZ : a.msmall;
   const int t0 = col % a.tiles0, t1 = col / a.tiles0;
   const int i00 = t0 * 32 + NGHOSTS, i10 = t1 * BY + NGHOSTS;
   const int N0 = a.N0, top = NGHOSTS + a.Nxx1, Nxx2 = a.Nxx2;
-  const int nz = min(zc, NGHOSTS + Nxx2 - z0);
+  const int nz = min(zc, Nxx2 - zf);
+  // substeps 2 and 4 sweep the planes the other way round: they start on the
+  // planes the substep before left in L2 (march_reversed)
+  const int z0 = NGHOSTS + (march_reversed(STAGE) ? Nxx2 - zf - nz : zf);
   // element offsets fit in 32 bits (march_fits), so every address is one
   // 32-bit offset scaled onto a base pointer
   const unsigned N01 = (unsigned)a.N01, Ntot = (unsigned)a.Ntot;
@@ -291,7 +300,7 @@ __global__ void __launch_bounds__(32 * BY, MINB)
   __shared__ bool last;
   pdl_enter();
   int lo = 0, hi = n - 1;
-  const int bx = blockIdx.x;
+  const int bx = march_reversed(STAGE) ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
     if (__ldg(offs + mid) <= bx)
