@@ -132,9 +132,12 @@ int nrpyell_get_step_mode(void);
  * away.  nrpyell_set_async(1) lets them return after enqueueing; the caller
  * then orders host access with nrpyell_synchronize(). */
 void nrpyell_set_async(int enable);
-/* Tile shape of the fused RK4 substep kernel.  By default the library times
- * every shape on the caller's grid the first time a grid size is stepped
- * and keeps the fastest.  nrpyell_set_tile(t) forces shape t (-1: autotune);
+/* Tile shape of the fused RK4 substep kernel.  By default the relaxation
+ * drivers run grids that fit on chip without these kernels (whole RK4 steps in
+ * one cooperative launch), and for the others, and in the step calls, the
+ * library times every shape on the caller's grid the first time a grid size is
+ * stepped and keeps the fastest.  nrpyell_set_tile(t) forces shape t, for
+ * every grid (-1: the default);
  * nrpyell_get_tile reports the shape in use for a grid (block 32 x by threads,
  * `planes` consecutive i2 planes per thread), -1 if not tuned yet; its fp32
  * argument selects FP64 (0), FP32 (1) or the FP32 correction form of

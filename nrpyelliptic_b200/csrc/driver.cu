@@ -330,13 +330,12 @@ template RelaxResult relax_loop<float>(const Dims&, RfmTables*, BcTables*, L2Tab
 template <typename T>
 RelaxResult relax_grid(const Dims& d, RfmTables* rt, BcTables* bt, L2Tables* lt, FusedWork* w, Scratch* s,
                        const StateBuffers& b, const RelaxParams& rp) {
-  if constexpr (sizeof(T) == 8) {
-    if (resident_ok<T>(d)) {
-      std::vector<RelaxResult> r;
-      const ResGrid g = {d, rt, bt, lt, b, rp, w->state, (rp.history_buf ? rp.history_buf : w->history) + rp.history_offset};
-      if (!relax_resident<T>({g}, &r)) return {0, false, NAN};
-      return r[0];
-    }
+  // FP32 runs in the correction form only
+  if ((sizeof(T) == 8 || b.R0) && resident_ok<T>(d)) {
+    std::vector<RelaxResult> r;
+    const ResGrid g = {d, rt, bt, lt, b, rp, w->state, (rp.history_buf ? rp.history_buf : w->history) + rp.history_offset};
+    if (!relax_resident<T>({g}, &r)) return {0, false, NAN};
+    return r[0];
   }
   const int tile = tuned_tile<T>(d, rt, bt, w, s, b, rp, lt);
   return relax_loop<T>(d, rt, bt, lt, w, s, tile, b, rp);

@@ -15,20 +15,29 @@
 //     and its neighbours read value and number with one load and keep what
 //     carries the number they wait for: no fence, no flag, no grid barrier,
 //     and a block waits only for the neighbours it reads;
+//   * twelve warps of a block compute and four fetch: the halos of the next
+//     substep arrive while this one is computed.  Both work through the planes
+//     in a lower and an upper half and meet at named barriers, so the compute
+//     warps start on the lower half while the upper halos are under way;
 //   * ghost points across xx0 = 0 and the axis are images of the block's own
 //     columns (the tile holds all planes), so inner boundaries cost nothing;
 //   * the radiation BC of the x0max face runs in blocks of its own beside the
-//     interior blocks, on the same arithmetic as column_rows;
+//     interior blocks, on the same arithmetic as column_rows; the ghost values
+//     that a column's next substep reads itself stay in the block;
 //   * at substep 1 each block publishes its share of the residual norm, and
 //     every block sums all shares in the same order before substep 4, which
 //     is the first one that overwrites y_n: three substeps hide the sum.
-// Every point is evaluated with the same device functions in the same order
-// as in the substep kernels, so the steps are bit-identical to theirs.
-// Measured per RK4 step (substep kernels -> here): 26.0 -> 11.5 us at 64x64x8,
-// 26.4 -> 14.6 at 90x75x10, 38.6 -> 25.3 at 128x128x16.  Bound by the exchange
-// (a store, one L2 round trip and the fetch's instructions: about 3700 of 5600
-// cycles of a substep at 64x64x8) and, from 96x96x12 on, by the instruction
-// issue and shared-memory loads of the interior blocks.
+// FP64 grids and the FP32 correction form run here.  Every point is evaluated
+// with the same device functions in the same order as in the substep kernels,
+// so the steps are bit-identical to theirs.
+// Measured per FP64 RK4 step (substep kernels -> here): 26.0 -> 12.0 us at
+// 64x64x8, 26.4 -> 15.7 at 90x75x10, 38.6 -> 23.5 at 128x128x16 (26.6 with all
+// warps fetching first and then computing); a 64x64x8 mixed relaxation 58.1 ->
+// 25.8 ms.  Bound by the exchange (a store, one L2 round trip and the fetch's
+// instructions: most of the 5600 cycles of a substep at 64x64x8) and, from
+// 96x96x12 on, by the instruction issue and shared-memory loads of the
+// interior blocks and by the radiation blocks' serial recurrence and gathers
+// (4400 + 5000 cycles of a substep at 128x128x16).
 //
 // Waits are bounded: a thread that polls too long raises the launch's error
 // flag, every block leaves at its next barrier and the host reports it.
@@ -45,8 +54,12 @@ namespace nrpyell {
 
 namespace {
 
-constexpr int kSlots = 4;            // substeps an exchanged value stays readable
-constexpr int kMaxThreads = 512;     // threads of a block; 256 for the tall columns (threads_of)
+constexpr int kSlots = 8;            // substeps an exchanged value stays readable
+// Threads of a block: in an interior block 384 compute (three warpgroups) and
+// 128 fetch halos.  The launch's 128 registers per thread are divided 144 : 80.
+constexpr int kThreads = 512, kCompute = 384;
+constexpr int kComputeRegs = 144, kFetchRegs = 80;
+static_assert(kCompute * kComputeRegs + (kThreads - kCompute) * kFetchRegs <= kThreads * 128, "registers of the launch");
 constexpr int kMaxBlocks = 160;      // interior blocks of one grid
 // radiation rows: 12 points at an odd pitch; planes are padded so that the rows
 // of the next plane continue the pattern of banks (13 (z R + row) mod 16)
@@ -88,9 +101,12 @@ struct Tagged<float> {
   }
 };
 
-// Threads of a block: 512 with up to 4 planes per thread (128 registers),
-// 256 with more (255 registers).
-__host__ __device__ constexpr int threads_of(int p) { return p <= 4 ? 512 : 256; }
+// Named barriers of an interior block (0 is __syncthreads).
+enum { kBarCompute = 1, kBarFree = 2, kBarFull = 4, kBarFetch = 8 };
+__device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(n) : "memory"); }
+__device__ __forceinline__ void bar_arrive(int id, int n) {
+  asm volatile("bar.arrive %0, %1;\n" ::"r"(id), "r"(n) : "memory");
+}
 
 // ---------------------------------------------------------------- geometry
 
@@ -115,10 +131,11 @@ __device__ __forceinline__ int opaque(int x) {
 
 __device__ __forceinline__ int split(int t, int n, int parts) { return (int)((long long)t * n / parts); }
 
-// Shared block state: the stop test's outcome, per-warp residual partials.
+// Shared block state: the stop test's outcome, whether a wait gave up, per-warp
+// residual partials.
 struct BlockState {
-  int stop;
-  double part[kMaxThreads / 32];
+  int stop, failed;
+  double part[kThreads / 32];
 };
 
 // Polls one tagged value until it carries `tag`; 1 when the wait gave up.
@@ -137,7 +154,7 @@ __device__ __forceinline__ int wait_tag(const typename Tagged<T>::Raw* p, unsign
 // version's slot and goes to tab[i].y of the shared buffer.  The table covers
 // all planes and is padded to whole units of 32 entries with copies of entry 0
 // that go to element 0 of the buffer, a corner that nothing reads.  Warp w
-// takes units w, w + nw, ...; up to four loads per thread are in flight, and a
+// takes units w, w + nw, ...; up to eight loads per thread are in flight, and a
 // batch counts only when every value of the warp carries the version (else one
 // lane waits for one missing value and the warp fetches the batch again).  The
 // instructions per entry are what this costs: with the offsets computed here
@@ -179,26 +196,32 @@ __device__ __forceinline__ int fetch(const int2* t, int stride, const typename T
   }
 }
 
-// Fetches one version of the halo; returns 1 when a wait gave up.
-template <typename T, typename D>
-__device__ __forceinline__ int gather(const ResJob<T>& J, const int2* tab, int units, unsigned ver, D* dst) {
-  const int nw = blockDim.x >> 5, warp = opaque(threadIdx.x >> 5);
+// Fetches the units of `tab` with warps w = 0 .. nw - 1; returns 1 when a wait
+// gave up.
+template <typename T, int NB, typename D>
+__device__ __forceinline__ int gather(const ResJob<T>& J, const int2* tab, int units, int w, int nw, unsigned ver,
+                                      D* dst) {
+  const int warp = opaque(w);
   const typename Tagged<T>::Raw* const slot =
       (const typename Tagged<T>::Raw*)J.xu + (long long)(ver & (kSlots - 1)) * J.xu_slot;
   int* const err = J.err;
   const int2* t = tab + warp * 32 + (threadIdx.x & 31);
   const int stride = nw * 32;
-  for (int n = units > warp ? (units - warp + nw - 1) / nw : 0; n > 0; n -= 4, t += 4 * stride) {
-    int failed;
-    switch (n) {
-      case 1: failed = fetch<T, 1>(t, stride, slot, ver, dst, err); break;
-      case 2: failed = fetch<T, 2>(t, stride, slot, ver, dst, err); break;
-      case 3: failed = fetch<T, 3>(t, stride, slot, ver, dst, err); break;
-      default: failed = fetch<T, 4>(t, stride, slot, ver, dst, err); break;
+  int n = units > warp ? (units - warp + nw - 1) / nw : 0;
+  for (; n >= NB; n -= NB, t += NB * stride)
+    if (fetch<T, NB>(t, stride, slot, ver, dst, err)) return 1;
+  if constexpr (NB > 4)
+    if (n >= 4) {
+      if (fetch<T, 4>(t, stride, slot, ver, dst, err)) return 1;
+      n -= 4;
+      t += 4 * stride;
     }
-    if (failed) return 1;
+  switch (n) {
+    case 1: return fetch<T, 1>(t, stride, slot, ver, dst, err);
+    case 2: return fetch<T, 2>(t, stride, slot, ver, dst, err);
+    case 3: return fetch<T, 3>(t, stride, slot, ver, dst, err);
+    default: return 0;
   }
-  return 0;
 }
 
 // One warp, before substep 4 of step n: the residual norm of y_n from all
@@ -263,32 +286,32 @@ __host__ __device__ inline int table_entries(int n, int Nz) { return ceil_div(n 
 
 // ---------------------------------------------------------- interior blocks
 
-template <typename T, bool CORR, int TX, int P>
+template <typename T, bool CORR, int TX, int P2>
 __device__ __forceinline__ void interior_block(const ResJob<T>& J, int local, unsigned base, int steps,
                                                unsigned char* smem, BlockState* bs) {
   using G = TileGeom<T, TX>;
   constexpr int PITCH = G::PITCH, RPW = G::RPW;
   using Raw = typename Tagged<T>::Raw;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, NT = blockDim.x;
-  const int Nz = J.Nxx2, N0 = J.N0;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int Nz = J.Nxx2, N0 = J.N0, Zh = (Nz + 1) / 2;  // planes of the lower half
   const int t0 = local % J.n0t, t1 = local / J.n0t;
   const int x0 = split(t0, J.Nxx0, J.n0t), w = split(t0 + 1, J.Nxx0, J.n0t) - x0;
   const int r0 = split(t1, J.Nxx1, J.n1t), h = split(t1 + 1, J.Nxx1, J.n1t) - r0;
   const int plane = (J.hmax + 2 * NGHOSTS) * PITCH;
-  int2* tab = reinterpret_cast<int2*>(smem);
-  T* const buf0 = reinterpret_cast<T*>(smem + sizeof(int2) * table_entries(10 * (J.hmax + TX), Nz));
+  int2* const tab = reinterpret_cast<int2*>(smem);
+  T* const buf0 = reinterpret_cast<T*>(smem + sizeof(int2) * (table_entries(10 * (J.hmax + TX), Nz) + 32));
   T* const buf1 = buf0 + (size_t)Nz * plane;
-  // source fields of the thread's points, [P][NF][FS]
-  constexpr int NF = CORR ? 5 : 3, FS = threads_of(P);
-  T* const fld = buf1 + (size_t)Nz * plane + tid;
   const bool left = t0 == 0, low = t1 == 0, high = t1 == J.n1t - 1;
-  // ---- halo entries: columns left and right, rows below and above
+  // ---- halo entries: columns left and right, rows below and above; the lower
+  // half's planes, then the upper half's, each in whole units
   const int xrow = J.xu_row;
   const int nl = left ? 0 : NGHOSTS * h, nr = NGHOSTS * h, nd = low ? 0 : NGHOSTS * w, nu = high ? 0 : NGHOSTS * w;
-  const int nent = nl + nr + nd + nu, units = ceil_div(nent * Nz, 32);
-  for (int i = tid; i < units * 32; i += NT) {
-    const bool pad = i >= nent * Nz;
-    const int z = pad ? 0 : i / nent;
+  const int nent = nl + nr + nd + nu, units0 = ceil_div(nent * Zh, 32), units1 = ceil_div(nent * (Nz - Zh), 32);
+  for (int u = tid; u < (units0 + units1) * 32; u += kThreads) {
+    const bool upper = u >= units0 * 32;
+    const int i = upper ? u - units0 * 32 : u;
+    const bool pad = i >= nent * (upper ? Nz - Zh : Zh);
+    const int z = pad ? 0 : (upper ? Zh : 0) + i / nent;
     int q = pad ? 0 : i % nent, jx, jr;
     if (q < nl) {
       jx = q % NGHOSTS - NGHOSTS;
@@ -304,13 +327,15 @@ __device__ __forceinline__ void interior_block(const ResJob<T>& J, int local, un
       jx = q % w;
       jr = h + q / w;
     }
-    tab[i] = make_int2((r0 + jr) * xrow + x0 + jx + z * J.xu_plane,
+    // padding: the half's first entry, to a corner of the tile
+    const int zp = pad && upper ? Zh : z;
+    tab[u] = make_int2((r0 + jr) * xrow + x0 + jx + zp * J.xu_plane,
                        pad ? 0 : (jr + NGHOSTS) * PITCH + jx + NGHOSTS + z * plane);
   }
   // ---- uu with its halo from y_n (corners of the tile are never read)
   {
     const int tw = w + 2 * NGHOSTS, th = h + 2 * NGHOSTS;
-    for (int e = tid; e < tw * th * Nz; e += NT) {
+    for (int e = tid; e < tw * th * Nz; e += kThreads) {
       const int xx = e % tw, q = e / tw, rr = q % th, z = q / th;
       int jx = xx - NGHOSTS, jr = rr - NGHOSTS;
       if ((jx < 0 || jx >= w) && (jr < 0 || jr >= h)) continue;
@@ -337,27 +362,72 @@ __device__ __forceinline__ void interior_block(const ResJob<T>& J, int local, un
           __ldcg(J.y + (jx + NGHOSTS) + (long long)N0 * (jr + NGHOSTS) + J.N01 * (zs + NGHOSTS));
     }
   }
-  // ---- the thread's column and its P planes
-  const int nrg = (J.hmax + RPW - 1) / RPW;
-  const int x = lane % TX, row = (warp % nrg) * RPW + lane / TX, z0 = (warp / nrg) * P;
-  const bool col_ok = x < w && row < h && z0 < Nz;
+  __syncthreads();
+
+  if (warp >= kCompute / 32) {
+    // ---- the fetching warps: the halo of every version after the first, half
+    // by half, into the buffer that version is read from
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(kFetchRegs));
+    const int gw = warp - kCompute / 32, ngw = (kThreads - kCompute) / 32;
+    const int n0 = J.n_start;
+    bool failed = false;
+    for (int i = 1; i < 4 * steps; i++) {
+      const unsigned ver = base + i;
+      const int par = i & 1;
+      T* const dst = par ? buf1 : buf0;
+      // the substep that read this buffer's previous version is done
+      if (i >= 2) bar_sync(kBarFree + par, kThreads);
+      if ((i & 3) == 3) {  // substep 4 comes: the stop test first
+        if (gw == ngw - 1 && !failed) failed = stop_test<T>(J, local, n0 + (i >> 2), ver - 2, bs);
+        if (failed && lane == 0) bs->failed = 1;
+        bar_sync(kBarFetch, kThreads - kCompute);
+        if (lane == 0 && gw == 0 && bs->failed) bs->stop = 1;
+        bar_sync(kBarFetch, kThreads - kCompute);
+        if (bs->stop) {
+          bar_arrive(kBarFull + par, kThreads);
+          break;
+        }
+      }
+      // a wait that gave up ends the launch at the next stop test; until then
+      // nothing is waited for
+      if (!failed) failed = gather<T, 8>(J, tab, units0, gw, ngw, ver, dst);
+      bar_arrive(kBarFull + par, kThreads);
+      if (!failed) failed = gather<T, 8>(J, tab + units0 * 32, units1, gw, ngw, ver, dst);
+      bar_arrive(kBarFull + 2 + par, kThreads);
+    }
+    return;
+  }
+
+  // ---- the computing warps: a thread's column and its P2 planes of either half
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(kComputeRegs));
+  constexpr int P = 2 * P2, NF = CORR ? 5 : 3;
+  T* const fld = buf1 + (size_t)Nz * plane + tid;  // source fields of the thread's points, [P][NF][kCompute]
+  const int nrg = (J.hmax + RPW - 1) / RPW, zg = warp / nrg;
+  const int x = lane % TX, row = (warp % nrg) * RPW + lane / TX, zlo = zg * P2;
+  const bool col_ok = x < w && row < h && zlo < Zh;
   const long long gcol = (x0 + x + NGHOSTS) + (long long)N0 * (r0 + row + NGHOSTS);
   const int scol = (row + NGHOSTS) * PITCH + x + NGHOSTS;
+  // plane of point p (p < P2: lower half), or -1
+  auto plane_of = [&](int p) -> int {
+    const int k = zlo + (p < P2 ? p : p - P2);
+    return p < P2 ? (k < Zh ? k : -1) : (k < Nz - Zh ? Zh + k : -1);
+  };
   T yu[P], yv[P], au[P], av[P], vv[P];
   T C22 = 0, C00 = 0, C11 = 0, C1 = 0, C0 = 0, Cc = 0;
 #pragma unroll
   for (int p = 0; p < P; p++) {
     yu[p] = yv[p] = au[p] = av[p] = vv[p] = (T)0;
-    if (col_ok && z0 + p < Nz) {
-      const long long g = gcol + J.N01 * (z0 + p + NGHOSTS);
+    const int z = plane_of(p);
+    if (col_ok && z >= 0) {
+      const long long g = gcol + J.N01 * (z + NGHOSTS);
       yu[p] = __ldcg(J.y + g);
       yv[p] = __ldcg(J.y + J.Ntot + g);
-      fld[(p * NF + 0) * FS] = __ldg(J.aux + ADD_TIMES_AUUGF * J.Ntot + g);
-      fld[(p * NF + 1) * FS] = __ldg(J.aux + PSI_BACKGROUNDGF * J.Ntot + g);
-      fld[(p * NF + 2) * FS] = __ldg(J.aux + WAVESPEEDGF * J.Ntot + g);
+      fld[(p * NF + 0) * kCompute] = __ldg(J.aux + ADD_TIMES_AUUGF * J.Ntot + g);
+      fld[(p * NF + 1) * kCompute] = __ldg(J.aux + PSI_BACKGROUNDGF * J.Ntot + g);
+      fld[(p * NF + 2) * kCompute] = __ldg(J.aux + WAVESPEEDGF * J.Ntot + g);
       if constexpr (CORR) {
-        fld[(p * NF + 3) * FS] = __ldg(J.R0 + g);
-        fld[(p * NF + 4) * FS] = __ldg(J.R0 + J.Ntot + g);
+        fld[(p * NF + 3) * kCompute] = __ldg(J.R0 + g);
+        fld[(p * NF + 4) * kCompute] = __ldg(J.R0 + J.Ntot + g);
       }
       vv[p] = yv[p];
     }
@@ -373,38 +443,43 @@ __device__ __forceinline__ void interior_block(const ResJob<T>& J, int local, un
   const bool img0 = left && x < NGHOSTS, imgd = low && row < NGHOSTS, imgu = high && row >= h - NGHOSTS;
   const bool image = img0 || imgd || imgu;
   const bool pub_v = x0 + x >= J.Nxx0 - 7;
-  const int xg = (r0 + row) * xrow + x0 + x;                      // exchange offset of the column, plane 0
+  const int xg = (r0 + row) * xrow + x0 + x;                              // exchange offset of the column, plane 0
   const int vg = J.xv0 + (r0 + row) * 12 + (x0 + x - (J.Nxx0 - 7));
   const T dt = J.dt, eta = J.eta;
-  const int xu_plane = J.xu_plane, nzp = Nz * plane;
-  const int himg = J.half2 * plane;
+  const int xu_plane = J.xu_plane, xv_plane = J.xv_plane, nzp = Nz * plane, himg = J.half2 * plane;
+  const long long xu_slot = J.xu_slot;
+  double r2 = 0.0;
 
-  auto substep = [&](auto st, const T* __restrict__ cur, T* __restrict__ nxt, unsigned ver) {
-    constexpr int STAGE = decltype(st)::value;
-    double r2 = 0.0;
-    if (col_ok) {
+  // one substep of the lower (H = 0) or upper half
+  auto substep = [&](auto st, auto half, const T* __restrict__ cur, T* __restrict__ nxt, unsigned ver) {
+    constexpr int STAGE = decltype(st)::value, H = decltype(half)::value;
+    if (STAGE == 1 && H == 0) r2 = 0.0;
+    const int zb = opaque(H ? Zh + zlo : zlo), zend = H ? Nz : Zh;
+    if (col_ok && zb < zend) {
       double wl2 = 0.0;
       if (STAGE == 1) wl2 = __ldg(J.w + gcol);
-      int o = opaque(z0 * plane);  // offset of the plane
-      const int sc = opaque(scol);
-      // uu along i2: planes z0-5 .. z0+P+4, wrapped (those past a partial last
+      int o = zb * plane;  // offset of the plane
+      const int oend = zend * plane, sc = opaque(scol);
+      // uu along i2: planes zb-5 .. zb+P2+4, wrapped (those past a partial last
       // chunk are loaded but not used)
-      T q[P + 10];
+      T q[P2 + 10];
       {
         int oq = o - NGHOSTS * plane;
         if (oq < 0) oq += nzp;
 #pragma unroll
-        for (int j = 0; j < P + 10; j++) {
+        for (int j = 0; j < P2 + 10; j++) {
           q[j] = cur[sc + oq];
           oq += plane;
           if (oq >= nzp) oq -= nzp;
         }
       }
-      const T* f = fld + opaque(0);
-      Raw* xu = (Raw*)J.xu + ((long long)((ver + 1) & (kSlots - 1)) * J.xu_slot + (xg + opaque(z0) * xu_plane));
+      const T* f = fld + opaque(H * P2 * NF * kCompute);
+      Raw* xu = (Raw*)J.xu + (long long)((ver + 1) & (kSlots - 1)) * xu_slot;
+      Raw* xv = xu + (vg + zb * xv_plane);
+      xu += xg + zb * xu_plane;
 #pragma unroll
-      for (int p = 0; p < P; p++) {
-        if (o < nzp) {
+      for (int p = 0; p < P2; p++) {
+        if (o < oend) {
           const T* c = cur + sc + o;
           T s0 = 0, s1 = 0, s00 = 0, s11 = 0, s22 = 0;
 #pragma unroll
@@ -419,28 +494,27 @@ __device__ __forceinline__ void interior_block(const ResJob<T>& J, int local, un
 #pragma unroll
           for (int k = 1; k <= 5; k++) s22 = fma(W<T>::e(k), q[p + 5 + k] + q[p + 5 - k], s22);
           T ku, kv, br;
-          const T* fp = f + p * NF * FS;
+          const T* fp = f + p * NF * kCompute;
+          constexpr int FS = kCompute;
+          const int i = H * P2 + p;
           if constexpr (CORR) {
             T ju, jv;
-            point_rhs_correction<T>(q[p + 5], vv[p], fp[0], fp[FS], fp[2 * FS], C22, C00, C11, C1, C0, Cc, s0, s1, s00,
+            point_rhs_correction<T>(q[p + 5], vv[i], fp[0], fp[FS], fp[2 * FS], C22, C00, C11, C1, C0, Cc, s0, s1, s00,
                                     s11, s22, eta, fp[3 * FS], fp[4 * FS], ku, kv, br, ju, jv);
           } else {
-            point_rhs<T>(q[p + 5], vv[p], fp[0], fp[FS], fp[2 * FS], C22, C00, C11, C1, C0, Cc, s0, s1, s00, s11, s22,
+            point_rhs<T>(q[p + 5], vv[i], fp[0], fp[FS], fp[2 * FS], C22, C00, C11, C1, C0, Cc, s0, s1, s00, s11, s22,
                          eta, ku, kv, br);
           }
           T ou, ov;
-          rk_combine<T, STAGE>(ku, yu[p], au[p], ou, dt);
-          rk_combine<T, STAGE>(kv, yv[p], av[p], ov, dt);
-          vv[p] = ov;
+          rk_combine<T, STAGE>(ku, yu[i], au[i], ou, dt);
+          rk_combine<T, STAGE>(kv, yv[i], av[i], ov, dt);
+          vv[i] = ov;
           if (STAGE == 4) {
-            yu[p] = ou;
-            yv[p] = ov;
+            yu[i] = ou;
+            yv[i] = ov;
           }
           Tagged<T>::store(xu, ou, ver + 1);
-          if (pub_v)
-            Tagged<T>::store((Raw*)J.xu + ((long long)((ver + 1) & (kSlots - 1)) * J.xu_slot +
-                                           (vg + (opaque(z0) + p) * J.xv_plane)),
-                             ov, ver + 1);
+          if (pub_v) Tagged<T>::store(xv, ov, ver + 1);
           T* n = nxt + sc + o;
           *n = ou;
           if (image) {  // images across xx0 = 0 and the axis: mirrored, half a turn on
@@ -456,49 +530,54 @@ __device__ __forceinline__ void interior_block(const ResJob<T>& J, int local, un
         }
         o += plane;
         xu += xu_plane;
+        xv += xv_plane;
       }
     }
-    if (STAGE == 1) {
+    if (STAGE == 1 && H == 1) {
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) r2 += __shfl_down_sync(0xffffffffu, r2, o);
+      for (int s = 16; s > 0; s >>= 1) r2 += __shfl_down_sync(0xffffffffu, r2, s);
       if (lane == 0) bs->part[warp] = r2;
     }
   };
-
-  unsigned ver = base;
+  // substep `st` of version base + i: its halves as their halos arrive, then
+  // every computing warp's values are written and the buffer read is free
+  auto full_substep = [&](auto st, int i) {
+    const int par = i & 1;
+    const T* cur = par ? buf1 : buf0;
+    T* nxt = par ? buf0 : buf1;
+    if (i > 0) bar_sync(kBarFull + par, kThreads);
+    if (decltype(st)::value == 4 && bs->stop) return true;
+    substep(st, std::integral_constant<int, 0>(), cur, nxt, base + i);
+    if (i > 0) bar_sync(kBarFull + 2 + par, kThreads);
+    substep(st, std::integral_constant<int, 1>(), cur, nxt, base + i);
+    bar_sync(kBarCompute, kCompute);
+    bar_arrive(kBarFree + par, kThreads);
+    return false;
+  };
   const int n0 = J.n_start;
   for (int k = 0; k < steps; k++) {
-    const int n = n0 + k;
-    if (__syncthreads_or(k > 0 ? gather<T>(J, tab, units, ver, buf0) : 0)) return;
-    substep(std::integral_constant<int, 1>(), buf0, buf1, ver);
-    ver++;
-    if (__syncthreads_or(gather<T>(J, tab, units, ver, buf1))) return;
+    full_substep(std::integral_constant<int, 1>(), 4 * k);
     if (warp == 0) {  // the block's share of the residual norm
-      double s = lane < (NT >> 5) ? bs->part[lane] : 0.0;
+      double s = lane < kCompute / 32 ? bs->part[lane] : 0.0;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-      if (lane == 0) Tagged<double>::store(J.part + (n & 1) * (J.n0t * J.n1t) + local, s, ver);
+      if (lane == 0)
+        Tagged<double>::store(J.part + ((n0 + k) & 1) * (J.n0t * J.n1t) + local, s, base + 4 * k + 1);
     }
-    substep(std::integral_constant<int, 2>(), buf1, buf0, ver);
-    ver++;
-    if (__syncthreads_or(gather<T>(J, tab, units, ver, buf0))) return;
-    substep(std::integral_constant<int, 3>(), buf0, buf1, ver);
-    ver++;
-    int failed = warp == (NT >> 5) - 1 ? stop_test<T>(J, local, n, ver - 2, bs) : 0;
-    failed |= gather<T>(J, tab, units, ver, buf1);
-    if (__syncthreads_or(failed)) return;
-    if (bs->stop) break;
-    substep(std::integral_constant<int, 4>(), buf1, buf0, ver);
-    ver++;
+    full_substep(std::integral_constant<int, 2>(), 4 * k + 1);
+    full_substep(std::integral_constant<int, 3>(), 4 * k + 2);
+    if (full_substep(std::integral_constant<int, 4>(), 4 * k + 3)) break;
   }
-  if (col_ok) {
+  if (col_ok && !bs->failed) {
 #pragma unroll
-    for (int p = 0; p < P; p++)
-      if (z0 + p < Nz) {
-        const long long g = gcol + J.N01 * (z0 + p + NGHOSTS);
+    for (int p = 0; p < P; p++) {
+      const int z = plane_of(p);
+      if (z >= 0) {
+        const long long g = gcol + J.N01 * (z + NGHOSTS);
         J.y[g] = yu[p];
         J.y[J.Ntot + g] = yv[p];
       }
+    }
   }
 }
 
@@ -530,7 +609,9 @@ __host__ __device__ inline RadLayout rad_layout(int R, int Nz) {
   l.total = l.w + 72;
   return l;
 }
-__host__ __device__ inline int rad_entries(int R) { return 2 * (12 * R + 6 * 2 * NGHOSTS); }
+// Entries of a plane: the last 7 interior points of the block's rows (their
+// ghost points stay in the block) and 6 points of the rows around them.
+__host__ __device__ inline int rad_entries(int R) { return 2 * (7 * R + 6 * 2 * NGHOSTS); }
 
 // Points jj0 .. jj0 + K - 1 of one column (q of its 2 RZ): f the column's row in
 // F, g its geometry, w the weights.  K points share the column's 12 values
@@ -589,18 +670,18 @@ __device__ __forceinline__ void radiation_block(const ResJob<T>& J, int local, u
   double* const fp = base_s + lay.fp;
   double* const geo = base_s + lay.geo;
   double* const wx0 = base_s + lay.w;
-  // ---- entries: 12 points of the block's rows, 6 of the rows around them,
-  // and the same points from y_n (ghost rows across the axis: half a turn on)
+  // ---- the entries, and the same points from y_n (ghost rows across the axis:
+  // half a turn on)
   const int xrow = J.xu_row;
   for (int i = tid; i < units * 32; i += NT) {
     const bool pad = i >= nent * Nz;
     const int z = pad ? 0 : i / nent, e = pad ? 0 : i % nent, g = e / (nent / 2);
     int q = e % (nent / 2), jr, c;
-    if (q < 12 * R) {
-      jr = q / 12;
-      c = q % 12;
+    if (q < 7 * R) {
+      jr = q / 7;
+      c = q % 7;
     } else {
-      q -= 12 * R;
+      q -= 7 * R;
       c = 6 + q % 6;
       q /= 6;
       jr = q < NGHOSTS ? q - NGHOSTS : R + q - NGHOSTS;
@@ -662,11 +743,26 @@ __device__ __forceinline__ void radiation_block(const ResJob<T>& J, int local, u
     acc[L] = (T)0;
     base_rhs[L] = (CORR && live) ? (double)__ldg(J.R0 + gidx + L) : 0.0;
   }
-  // a warp's derivative task: K = 1, 2, 3 or 6 points (the smallest K whose
-  // tasks leave a warp to the others) of 32 of both gridfunctions' columns;
-  // the RHS of the last interior points goes to the warps left
+  double* const own = F + cg * gplane + cz * plane + (crow + NGHOSTS) * kRadPitch + 7;  // its ghost points in F
+  if (live)
+    for (int L = 0; L < NGHOSTS; L++) own[L] = (double)y[L];
+  // a warp's derivative task: K = 1, 2, 3 or 6 points of 32 of both
+  // gridfunctions' columns; the RHS of the last interior points goes to the
+  // warps left, in rounds that take about twice a point's time: the K with the
+  // shortest longer one
   const int nw = NT >> 5, n_rhs = ceil_div(RZ, 32), n_col = ceil_div(2 * RZ, 32);
-  const int K = 6 * n_col < nw ? 1 : 3 * n_col < nw ? 2 : 2 * n_col < nw ? 3 : 6;
+  int K = 6;
+  {
+    int best = 1 << 30;
+    for (int k = 6; k >= 1; k = k == 6 ? 3 : k - 1) {
+      const int left = nw - n_col * (6 / k);
+      const int t = left > 0 ? max(k, 2 * ceil_div(n_rhs, left)) : left == 0 ? k + 2 * ceil_div(n_rhs, nw) : 1 << 30;
+      if (t <= best) {
+        best = t;
+        K = k;
+      }
+    }
+  }
   const int n_drf = n_col * (6 / K), rest = nw - n_drf;
   const int jj0 = warp / n_col * K, drf_q = (warp % n_col) * 32 + (tid & 31);
   const bool drf_on = warp < n_drf && drf_q < 2 * RZ;
@@ -733,6 +829,7 @@ __device__ __forceinline__ void radiation_block(const ResJob<T>& J, int local, u
       const double* const g = geo + opaque(crow * kGeoStride);
       double k = kl[t];
       Raw* to = to0 + (long long)((ver + 1) & (kSlots - 1)) * slot;
+      double mine[NGHOSTS];
 #pragma unroll
       for (int L = 0; L < NGHOSTS; L++) {
         k = radiation_layer(cw, k, X[L * 2 * RZ + t], Y[L * 2 * RZ + t], g[24 + L], g[19 + L]);
@@ -741,7 +838,12 @@ __device__ __forceinline__ void radiation_block(const ResJob<T>& J, int local, u
         rk_combine<T, STAGE>((T)kfull, y[L], acc[L], ou, dt);
         if (STAGE == 4) y[L] = ou;
         Tagged<T>::store(to + L, ou, ver + 1);
+        mine[L] = (double)ou;
       }
+      // after the recurrence, whose loads the compiler would keep behind these
+      // (this substep's reads of F are done: the barrier above)
+#pragma unroll
+      for (int L = 0; L < NGHOSTS; L++) own[L] = mine[L];
     }
   };
 
@@ -749,17 +851,17 @@ __device__ __forceinline__ void radiation_block(const ResJob<T>& J, int local, u
   const int n0 = J.n_start;
   for (int k = 0; k < steps; k++) {
     const int n = n0 + k;
-    if (__syncthreads_or(k > 0 ? gather<T>(J, tab, units, ver, F) : 0)) return;
+    if (__syncthreads_or(k > 0 ? gather<T, 4>(J, tab, units, warp, NT >> 5, ver, F) : 0)) return;
     substep(std::integral_constant<int, 1>(), ver);
     ver++;
-    if (__syncthreads_or(gather<T>(J, tab, units, ver, F))) return;
+    if (__syncthreads_or(gather<T, 4>(J, tab, units, warp, NT >> 5, ver, F))) return;
     substep(std::integral_constant<int, 2>(), ver);
     ver++;
-    if (__syncthreads_or(gather<T>(J, tab, units, ver, F))) return;
+    if (__syncthreads_or(gather<T, 4>(J, tab, units, warp, NT >> 5, ver, F))) return;
     substep(std::integral_constant<int, 3>(), ver);
     ver++;
     int failed = warp == (NT >> 5) - 1 ? stop_test<T>(J, local, n, ver - 2, bs) : 0;
-    failed |= gather<T>(J, tab, units, ver, F);
+    failed |= gather<T, 4>(J, tab, units, warp, NT >> 5, ver, F);
     if (__syncthreads_or(failed)) return;
     if (bs->stop) break;
     substep(std::integral_constant<int, 4>(), ver);
@@ -774,8 +876,8 @@ __device__ __forceinline__ void radiation_block(const ResJob<T>& J, int local, u
 // Up to `steps` RK4 steps of every job; block b belongs to the last job with
 // cta0 <= b.  Exchanged values of this launch carry tags base + 1 ..
 // base + 4 steps.
-template <typename T, bool CORR, int TX, int P>
-__global__ void __launch_bounds__(threads_of(P), 1)
+template <typename T, bool CORR, int TX, int P2>
+__global__ void __launch_bounds__(kThreads, 1)
     k_relax_resident(const ResJob<T>* __restrict__ jobs, int njobs, unsigned base, int steps) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ BlockState bs;
@@ -788,12 +890,13 @@ __global__ void __launch_bounds__(threads_of(P), 1)
     J = jobs[j];
     J.n_start = J.state[0];
     bs.stop = J.state[1];
+    bs.failed = 0;
   }
   __syncthreads();
   if (bs.stop) return;  // done before this launch
   const int local = (int)blockIdx.x - J.cta0;
   if (local < J.n0t * J.n1t)
-    interior_block<T, CORR, TX, P>(J, local, base, steps, smem, &bs);
+    interior_block<T, CORR, TX, P2>(J, local, base, steps, smem, &bs);
   else
     radiation_block<T, CORR>(J, local, base, steps, smem, &bs);
 }
@@ -817,7 +920,7 @@ int device_attr(cudaDeviceAttr a) {
 int tile_pitch(bool fp64, int tx) { return fp64 ? (tx == 8 ? 24 : 26) : (tx == 8 ? 24 : 48); }
 
 constexpr int kTX[] = {8, 16};
-constexpr int kP[] = {1, 2, 4, 6, 8};
+constexpr int kP[] = {1, 2, 3};  // planes of a thread per half
 
 template <typename T>
 using ResKernel = void (*)(const ResJob<T>*, int, unsigned, int);
@@ -827,8 +930,8 @@ ResKernel<T> resident_kernel(int tx, int p) {
   constexpr bool CORR = sizeof(T) == 4;
 #define NRPYELL_RES(TX, P) \
   if (tx == TX && p == P) return k_relax_resident<T, CORR, TX, P>;
-  NRPYELL_RES(8, 1) NRPYELL_RES(8, 2) NRPYELL_RES(8, 4) NRPYELL_RES(8, 6) NRPYELL_RES(8, 8)
-  NRPYELL_RES(16, 1) NRPYELL_RES(16, 2) NRPYELL_RES(16, 4) NRPYELL_RES(16, 6) NRPYELL_RES(16, 8)
+  NRPYELL_RES(8, 1) NRPYELL_RES(8, 2) NRPYELL_RES(8, 3)
+  NRPYELL_RES(16, 1) NRPYELL_RES(16, 2) NRPYELL_RES(16, 3)
 #undef NRPYELL_RES
   return nullptr;
 }
@@ -890,7 +993,7 @@ bool ensure_resident(size_t bytes, size_t jobs_bytes, size_t pinned_ints) {
 // RK4 steps of one launch: long enough that loading and storing the state
 // (a few us) does not show, short enough that a launch ends within
 // milliseconds.
-constexpr int kStepsPerLaunch = 256;
+constexpr int kStepsPerLaunch = 512;
 
 }  // namespace
 
@@ -927,29 +1030,25 @@ ResPlan resident_plan(const Dims& d, int max_blocks) {
       const int R = ceil_div(d.Nxx1, nrad);
       if (n0t * n1t > kMaxBlocks) continue;
       for (int p : kP) {
-        const int warps = nrg * ceil_div(Nz, p);
-        // all warps a block can have: those without points still fetch
-        const int threads = threads_of(p);
-        if (std::max(warps * 32, 2 * R * Nz) > threads) continue;
-        const size_t s_int = sizeof(int2) * table_entries(10 * (hmax + tx), Nz) +
-                             sizeof(T) * ((size_t)2 * Nz * (hmax + 2 * NGHOSTS) * tile_pitch(fp64, tx) + (size_t)nf * p * threads_of(p));
+        if (nrg * ceil_div((Nz + 1) / 2, p) > kCompute / 32 || 2 * R * Nz > kThreads) continue;
+        const size_t s_int = sizeof(int2) * (table_entries(10 * (hmax + tx), Nz) + 32) +
+                             sizeof(T) * ((size_t)2 * Nz * (hmax + 2 * NGHOSTS) * tile_pitch(fp64, tx) + (size_t)nf * 2 * p * kCompute);
         const size_t s_rad = sizeof(int2) * table_entries(rad_entries(R), Nz) + sizeof(double) * (size_t)rad_layout(R, Nz).total;
         const size_t smem = std::max(s_int, s_rad);
         if (smem > limit) continue;
         // cycles: the block's warps share the pipes (interior: shared-memory
-        // wavefronts, two per FP64 load of the 24 + 14 / P a point takes), and
-        // a fetch costs a round trip per eight loads of a thread
+        // wavefronts, two per FP64 load of the 24 + 10 / p a point takes), its
+        // fetches run beside that; a radiation block fetches, then computes
         const double pts = (double)std::min(tx, d.Nxx0) * hmax * Nz;
-        const double c_int = 700.0 + 300.0 * p + pts / 32.0 * (fp64 ? 2.0 : 1.0) * (24.0 + 14.0 / p) +
-                             700.0 * ceil_div(table_entries(10 * (hmax + tx), Nz), 4 * threads) +
-                             8.0 * table_entries(10 * (hmax + tx), Nz) / 32.0;
-        const double c_rad = 1000.0 + 500.0 * ceil_div(2 * ceil_div(2 * R * Nz, 32), threads / 32) +
-                             700.0 * ceil_div(table_entries(rad_entries(R), Nz), 4 * threads) +
+        const double c_int = 1200.0 + 500.0 * p + pts / 32.0 * (fp64 ? 2.0 : 1.0) * (28.0 + 10.0 / p);
+        const double fetch = 800.0 + 300.0 * ceil_div(table_entries(10 * (hmax + tx), Nz), 8 * (kThreads - kCompute));
+        const double c_rad = 1800.0 + 500.0 * ceil_div(2 * ceil_div(2 * R * Nz, 32), kThreads / 32) +
+                             700.0 * ceil_div(table_entries(rad_entries(R), Nz), 4 * kThreads) +
                              8.0 * table_entries(rad_entries(R), Nz) / 32.0;
-        const double cost = std::max(c_int, c_rad) + 0.1 * (n0t * n1t + nrad);
+        const double cost = std::max(std::max(c_int, fetch), c_rad) + 0.1 * (c_int + fetch + c_rad);
         if (cost < best_cost) {
           best_cost = cost;
-          best = {tx, p, threads, n0t, n1t, nrad, hmax, n0t * n1t + nrad, smem};
+          best = {tx, p, kThreads, n0t, n1t, nrad, hmax, n0t * n1t + nrad, smem, cost};
         }
       }
     }
@@ -957,12 +1056,31 @@ ResPlan resident_plan(const Dims& d, int max_blocks) {
   return best;
 }
 template ResPlan resident_plan<double>(const Dims&, int);
+template ResPlan resident_plan<float>(const Dims&, int);
 
 template <typename T>
 bool resident_ok(const Dims& d) {
   return g_forced_tile < 0 && resident_plan<T>(d, device_attr(cudaDevAttrMultiProcessorCount)).blocks > 0;
 }
 template bool resident_ok<double>(const Dims&);
+template bool resident_ok<float>(const Dims&);
+
+// How many grids of these dimensions share the SMs best, and the estimated
+// cycles of a substep per grid (0 grids: they do not fit).  More grids at once
+// leave each fewer blocks, but their exchanges overlap.
+template <typename T>
+ResTeam resident_team(const Dims& d, int available) {
+  ResTeam best = {0, 0.0};
+  const int sms = device_attr(cudaDevAttrMultiProcessorCount);
+  for (int m = 1; m <= std::min(available, 16); m++) {
+    const ResPlan p = resident_plan<T>(d, sms / m);
+    if (p.blocks == 0) continue;
+    if (best.grids == 0 || p.cost / m < best.cycles) best = {m, p.cost / m};
+  }
+  return best;
+}
+template ResTeam resident_team<double>(const Dims&, int);
+template ResTeam resident_team<float>(const Dims&, int);
 
 template <typename T>
 bool relax_resident(const std::vector<ResGrid>& grids, std::vector<RelaxResult>* results) {
@@ -1052,10 +1170,12 @@ bool relax_resident(const std::vector<ResGrid>& grids, std::vector<RelaxResult>*
   if (!status_ok()) return false;
   const ResJob<T>* jobs_dev = (const ResJob<T>*)g_res.jobs;
   int njobs = n;
-  // max_steps + 1 evaluations, and one launch more that only reads the done flags
-  const long long max_launches = (long long)max_steps / kStepsPerLaunch + 2;
-  for (long long k = 0; k < max_launches; k++) {
-    int steps = kStepsPerLaunch;
+  // max_steps + 1 residuals are evaluated at most; the states of a launch are
+  // read while the next one runs
+  long long left = (long long)max_steps + 1;
+  for (long long k = 0; left > 0; k++) {
+    int steps = (int)std::min<long long>(kStepsPerLaunch, left);
+    left -= steps;
     if (g_res.version > 0xf0000000u) {  // tags are about to wrap: start again from cleared slots
       NRPYELL_CUDA(cudaMemsetAsync(g_res.mem, 0, g_res.bytes, stream()));
       g_res.version = 0;
@@ -1106,5 +1226,6 @@ bool relax_resident(const std::vector<ResGrid>& grids, std::vector<RelaxResult>*
   return status_ok();
 }
 template bool relax_resident<double>(const std::vector<ResGrid>&, std::vector<RelaxResult>*);
+template bool relax_resident<float>(const std::vector<ResGrid>&, std::vector<RelaxResult>*);
 
 }  // namespace nrpyell

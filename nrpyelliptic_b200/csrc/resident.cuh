@@ -57,6 +57,7 @@ struct ResGrid {
 struct ResPlan {
   int tx, p, threads, n0t, n1t, nrad, hmax, blocks;
   size_t smem;
+  double cost;  // estimated cycles of a substep
 };
 template <typename T>
 ResPlan resident_plan(const Dims& d, int max_blocks);
@@ -65,8 +66,15 @@ ResPlan resident_plan(const Dims& d, int max_blocks);
 template <typename T>
 bool resident_ok(const Dims& d);
 
-// Relaxes the grids together in launches of many RK4 steps; results[i] as
-// relax_loop's.  Returns false on error.
+struct ResTeam {
+  int grids;
+  double cycles;
+};
+template <typename T>
+ResTeam resident_team(const Dims& d, int available);
+
+// Relaxes the grids, all of the same dimensions, together in launches of many
+// RK4 steps; results[i] as relax_loop's.  Returns false on error.
 template <typename T>
 bool relax_resident(const std::vector<ResGrid>& grids, std::vector<RelaxResult>* results);
 

@@ -48,9 +48,9 @@ def _relax(lib, prob, tile, call):
     return rc, steps.value, fin.value, hist, y, launches
 
 
-def _compare(lib, prob, call, max_launches):
+def _compare(lib, prob, call, max_launches, tile=SUBSTEP_TILE):
     a = _relax(lib, prob, -1, call)
-    b = _relax(lib, prob, SUBSTEP_TILE, call)
+    b = _relax(lib, prob, tile, call)
     assert a[5] <= max_launches < b[5] or b[1] < 4, (a[5], b[5])  # the on-chip form ran
     assert a[:2] == b[:2]
     np.testing.assert_allclose(a[3], b[3], rtol=0, atol=2e-11)
@@ -97,3 +97,23 @@ def test_rest_pair_takes_no_step(lib):
 
     a = _compare(lib, prob, relax, 4)
     assert a[0] == 0 and a[1] == 0
+
+
+MARCH_TILE = 20  # a marching shape: runs the FP32 correction form too
+
+
+@pytest.mark.parametrize("grid", [(12, 5, 6), (33, 40, 12), (64, 64, 8), (90, 75, 10), (128, 128, 16)])
+@pytest.mark.parametrize("switch", [-30.0, -4.0])
+def test_correction_form_matches_substep_kernels(lib, grid, switch):
+    """The FP32 correction form on chip: stretches of 48 steps and a shorter
+    last one, and the switch to FP64."""
+    prob = Problem(with_grid(sample_sweep(3)[1], grid), lib=lib)
+
+    def call(ds, n, fin, hist):
+        n32, n64 = C.c_int(0), C.c_int(0)
+        rc = lib.nrpyell_relax_mixed(C.byref(ds.g), prob.dt, -12.0, switch, 48, 130, prob.cfg.R_L2, C.byref(n32),
+                                     C.byref(n64), C.byref(fin), ptr(hist))
+        n.value = 1000 * n32.value + n64.value
+        return rc
+
+    _compare(lib, prob, call, 60, MARCH_TILE)
