@@ -301,10 +301,11 @@ int nrpyell_initial_lapse(const paramstruct *params, int npts, const REAL *xyz, 
 /* Batched relaxation: n configurations, each a griddata_struct set up as for
  * nrpyell_relax (its own grid size, parameters, bc_struct, rfm_struct and
  * device gridfunctions; dt[c] its time step), relaxed together from their
- * y_n_gfs to log10 L2 <= log10_tol or max_steps.  Every RK4 substep of all
- * configurations is one kernel launch (a shared-memory planes or marching
- * shape, autotuned on the batch or forced by nrpyell_set_tile); each
- * configuration stops on its own.
+ * y_n_gfs to log10 L2 <= log10_tol or max_steps.  Configurations for which it
+ * is faster relax on chip, several of equal grids in one cooperative launch
+ * (unless nrpyell_set_tile forces a shape); every RK4 substep of all others is
+ * one kernel launch (a shared-memory planes or marching shape, autotuned on
+ * the batch or forced).  Each configuration stops on its own.
  * steps_taken[c] and final_log10_l2[c] as in nrpyell_relax.  Returns the
  * number of configurations that did not converge (0: all did), < 0 on
  * error. */
@@ -315,8 +316,8 @@ int nrpyell_relax_batch(int n, griddata_struct *grids, const REAL *dt, REAL log1
  * FP32 correction stretch of up to fold_every steps or to log10_switch, the
  * fold; FP64 steps from the switch on), and the stretches of all
  * configurations still in the FP32 phase, then their FP64 phases, run as
- * batches (marching shapes for the FP32 stretches).  With the same tile
- * shapes each configuration's result is bitwise that of nrpyell_relax_mixed.
+ * batches (on chip, or marching shapes for the FP32 stretches).  With the same
+ * tile shapes each configuration's result is bitwise that of nrpyell_relax_mixed.
  * steps_fp32[c], steps_fp64[c], final_log10_l2[c] as there (each array may
  * be NULL); the FP32 buffers (13 Ntot floats per configuration) stay
  * allocated for later calls until nrpyell_release_tables.  Returns the number

@@ -1,5 +1,6 @@
 // Batched relaxation: many puncture configurations, on grids of different
-// sizes, relaxed together.  Every RK4 substep of all configurations is one
+// sizes, relaxed together.  Grids that run faster on chip (kernels_resident.cu)
+// go there, in teams of equal grids.  Every RK4 substep of all others is one
 // launch of the shared-memory planes or marching kernel
 // (k_substep_planes_batch, k_substep_march_batch): the
 // launch's blocks are the concatenated column blocks and interior tiles of
@@ -13,6 +14,7 @@
 #include <vector>
 
 #include "driver.cuh"
+#include "resident.cuh"
 #include "substep.cuh"
 
 namespace nrpyell {
@@ -156,13 +158,93 @@ struct BatchResult {
   std::vector<double> last;
 };
 
-// Relaxes the grids of gs together, each with its own RelaxParams (dt,
-// tolerance, max_steps); *tile: the tile shape, -1 = the forced one or the
-// fastest on this batch (set on return).  corr: FP32 correction form (every
-// grid's b.R0 set).  The results come from the device states and histories.
+// Microseconds per RK4 step of one grid on chip, in teams of grids of its
+// dimensions (kernels_resident.cu); 0: it does not fit.  A substep takes
+// about 1.8 times the cycles that the plan estimates (measured from 64x64x8 to
+// 128x128x16), at 1.9 GHz.
 template <typename T>
-bool run_batch(const std::vector<Grid>& gs, bool corr, int* tile, BatchResult* out) {
+double resident_us(const Dims& d, int count, int* team) {
+  const ResTeam t = resident_team<T>(d, count);
+  *team = t.grids;
+  return t.grids ? 4.0 * t.cycles * 1.8 / 1900.0 : 0.0;
+}
+
+// Relaxes on chip the grids for which that is faster than their share of the
+// batched launches, team after team, and marks them in `done`.  Batched
+// launches run at about 6.5 G (FP64) and 10 G (FP32 correction form) points x
+// RK4 steps per second, but not below 26 us a step.  Measured per grid and
+// step at 128x128x16: 24 us on chip, 40 us in a batch (FP64).  256 steps of
+// twelve grids of 96x96x12, 128x128x16 and 192x192x24, all in batched launches ->
+// by this rule: 201 -> 171 ms; 512 steps of sixteen 128x128x16 grids in the
+// correction form: 213 -> 189 ms.
+template <typename T>
+bool run_resident(const std::vector<Grid>& gs, std::vector<char>* done, BatchResult* out) {
   const int n = (int)gs.size();
+  const double points_per_us = sizeof(T) == 8 ? 6500.0 : 10000.0;
+  done->assign(n, 0);
+  auto points = [](const Dims& d) { return (double)d.Nxx0 * d.Nxx1 * d.Nxx2; };
+  struct Class {
+    std::vector<int> grids;
+    int team;
+    double us;
+  };
+  std::vector<Class> classes;
+  double batch_us = 0.0, chip_us = 0.0;
+  bool all = true;
+  for (int c = 0; c < n; c++) {
+    const Dims& d = gs[c].d;
+    Class* k = nullptr;
+    for (Class& q : classes)
+      if (memcmp(&gs[q.grids[0]].d, &d, sizeof(Dims)) == 0) k = &q;
+    if (!k) {
+      classes.push_back(Class());
+      k = &classes.back();
+    }
+    k->grids.push_back(c);
+    batch_us += points(d) / points_per_us;
+  }
+  for (Class& k : classes) {
+    k.us = resident_us<T>(gs[k.grids[0]].d, (int)k.grids.size(), &k.team);
+    all = all && k.team > 0;
+    chip_us += k.us * k.grids.size();
+  }
+  all = all && chip_us < std::max(26.0, batch_us);
+  for (const Class& k : classes) {
+    if (k.team == 0 || !(all || k.us < points(gs[k.grids[0]].d) / points_per_us)) continue;
+    for (size_t at = 0; at < k.grids.size(); at += k.team) {
+      std::vector<ResGrid> team;
+      for (size_t i = at; i < std::min(k.grids.size(), at + k.team); i++) {
+        const int c = k.grids[i];
+        const Grid& G = gs[c];
+        team.push_back({G.d, G.rt, G.bt, G.lt, G.b, G.rp, g_batch.state + kStateInts * c,
+                        g_batch.history + (size_t)c * g_batch.hist_len});
+      }
+      std::vector<RelaxResult> r;
+      if (!relax_resident<T>(team, &r)) return false;
+      for (size_t i = 0; i < r.size(); i++) {
+        const int c = k.grids[at + i];
+        (*done)[c] = 1;
+        out->steps[c] = r[i].steps;
+        out->converged[c] = r[i].converged;
+        out->last[c] = r[i].last_log10_l2;
+      }
+    }
+  }
+  return true;
+}
+
+// Relaxes the grids of gs, each with its own RelaxParams (dt, tolerance,
+// max_steps): on chip where that is faster (no tile forced), the others
+// together; *tile: the tile shape, -1 = the forced one or the fastest on this
+// batch (set on return).  corr: FP32 correction form (every grid's b.R0 set).
+// The results come from the device states and histories.
+template <typename T>
+bool run_batch(const std::vector<Grid>& gs, bool corr, int* tile, BatchResult* out);
+
+template <typename T>
+bool run_batched_launches(const std::vector<Grid>& gs, bool corr, int* tile, BatchResult* out) {
+  const int n = (int)gs.size();
+  if (n == 0) return true;
   int max_steps = 0, max_tiles = 0;
   bool fits = true;
   for (const Grid& G : gs) {
@@ -271,6 +353,38 @@ bool run_batch(const std::vector<Grid>& gs, bool corr, int* tile, BatchResult* o
                             cudaMemcpyDeviceToHost));
   }
   return status_ok();
+}
+
+template <typename T>
+bool run_batch(const std::vector<Grid>& gs, bool corr, int* tile, BatchResult* out) {
+  const int n = (int)gs.size();
+  if (g_forced_tile >= 0) return run_batched_launches<T>(gs, corr, tile, out);
+  int max_steps = 0, max_tiles = 0;
+  for (const Grid& G : gs) {
+    max_steps = std::max(max_steps, G.rp.max_steps);
+    max_tiles = std::max(max_tiles, max_interior_blocks(G.d));
+  }
+  if (!ensure_batch(n, max_steps + 1, max_tiles)) return false;
+  out->steps.assign(n, 0);
+  out->converged.assign(n, 0);
+  out->last.assign(n, NAN);
+  std::vector<char> done;
+  if (!run_resident<T>(gs, &done, out)) return false;
+  std::vector<Grid> rest;
+  std::vector<int> at;
+  for (int c = 0; c < n; c++)
+    if (!done[c]) {
+      rest.push_back(gs[c]);
+      at.push_back(c);
+    }
+  BatchResult r;
+  if (!run_batched_launches<T>(rest, corr, tile, &r)) return false;
+  for (size_t i = 0; i < at.size(); i++) {
+    out->steps[at[i]] = r.steps[i];
+    out->converged[at[i]] = r.converged[i];
+    out->last[at[i]] = r.last[i];
+  }
+  return true;
 }
 
 // Grids of a batched call, checked; rc 0, -1 (bad arguments or a CUDA

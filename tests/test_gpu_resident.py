@@ -117,3 +117,34 @@ def test_correction_form_matches_substep_kernels(lib, grid, switch):
         return rc
 
     _compare(lib, prob, call, 60, MARCH_TILE)
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+def test_batches_match_single_runs(lib, mixed):
+    """Batches whose grids run on chip, in teams of equal grids and with a team
+    cut short, beside grids too large for it: every grid's steps and solution
+    are those of its own run."""
+    from nrpyelliptic_b200.batch import relax_batch, relax_batch_mixed
+    grids = [(24, 17, 8)] * 3 + [(128, 128, 16)] * 2 + [(160, 160, 20)] + [(64, 64, 8)] * 5
+    probs = [Problem(with_grid(c, g), lib=lib) for c, g in zip(sample_sweep(len(grids)), grids)]
+    if mixed:
+        _, s32, s64, fin, states = relax_batch_mixed(probs, tol=-5.0, switch=-4.0, fold_every=100, max_steps=250, lib=lib)
+        steps = s32 * 1000 + s64
+    else:
+        _, steps, fin, states = relax_batch(probs, tol=-5.0, max_steps=250, lib=lib)
+    for i, p in enumerate(probs):
+
+        def call(ds, n, f, hist):
+            if not mixed:
+                return lib.nrpyell_relax(C.byref(ds.g), p.dt, -5.0, 250, p.cfg.R_L2, C.byref(n), C.byref(f), None)
+            n32, n64 = C.c_int(0), C.c_int(0)
+            rc = lib.nrpyell_relax_mixed(C.byref(ds.g), p.dt, -5.0, -4.0, 100, 250, p.cfg.R_L2, C.byref(n32),
+                                         C.byref(n64), C.byref(f), None)
+            n.value = 1000 * n32.value + n64.value
+            return rc
+
+        one = _relax(lib, p, -1, call)
+        assert one[1] == steps[i], grids[i]
+        np.testing.assert_allclose(fin[i], one[2], rtol=0, atol=2e-11)
+        np.testing.assert_array_equal(states[i].download("y_n"), one[4], err_msg=str(grids[i]))
+        states[i].free()
