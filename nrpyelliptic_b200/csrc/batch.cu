@@ -81,7 +81,7 @@ bool ensure_batch(int n, int hist_len, int partials_per) {
   NRPYELL_CUDA(dev_alloc(&g_batch.tickets, sizeof(unsigned int) * n));
   NRPYELL_CUDA(dev_alloc(&g_batch.offs, sizeof(int) * n));
   NRPYELL_CUDA(dev_alloc(&g_batch.devs, sizeof(SubDev<double>) * 5 * n));
-  NRPYELL_CUDA(cudaMemset(g_batch.tickets, 0, sizeof(unsigned int) * n));
+  NRPYELL_CUDA(cudaMemsetAsync(g_batch.tickets, 0, sizeof(unsigned int) * n, stream()));
   NRPYELL_CUDA(cudaMallocHost(&g_batch.pinned, sizeof(int) * kStateInts * n * 2));
   return status_ok();
 }

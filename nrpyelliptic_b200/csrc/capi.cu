@@ -693,7 +693,7 @@ int nrpyell_relax_mixed(griddata_struct* g, const REAL dt, const REAL log10_tol,
     NRPYELL_CUDA(cudaStreamSynchronize(stream()));
     if (!status_ok()) return -1;
     l2 = log10(1e-16 + sqrt(sum / su.lt->volume));
-    NRPYELL_CUDA(cudaMemcpy(w->history + n, &l2, sizeof(double), cudaMemcpyHostToDevice));
+    NRPYELL_CUDA(cudaMemcpyAsync(w->history + n, &l2, sizeof(double), cudaMemcpyHostToDevice, stream()));
     if (l2 <= log10_tol) {
       converged = true;
       break;

@@ -35,7 +35,7 @@ FusedWork* get_work(const Dims& d, int history_len) {
   w->f32 = nullptr;
   w->cycle_history = nullptr;
   NRPYELL_CUDA(dev_alloc(&w->state, sizeof(int) * 8 + sizeof(double) * 4));
-  NRPYELL_CUDA(cudaMemset(w->state, 0, sizeof(int) * 8 + sizeof(double) * 4));
+  NRPYELL_CUDA(cudaMemsetAsync(w->state, 0, sizeof(int) * 8 + sizeof(double) * 4, stream()));
   w->zero_flag = w->state + 4;
   w->history_len = history_len > 16 ? history_len : 16;
   NRPYELL_CUDA(dev_alloc(&w->history, sizeof(double) * w->history_len));

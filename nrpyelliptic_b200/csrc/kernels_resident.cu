@@ -955,7 +955,7 @@ size_t align_up(size_t n) { return (n + 255) / 256 * 256; }
 bool ensure_resident(size_t bytes, size_t jobs_bytes, size_t pinned_ints) {
   if (!g_res.err) {
     NRPYELL_CUDA(dev_alloc(&g_res.err, sizeof(int)));
-    NRPYELL_CUDA(cudaMemset(g_res.err, 0, sizeof(int)));
+    NRPYELL_CUDA(cudaMemsetAsync(g_res.err, 0, sizeof(int), stream()));
     for (cudaEvent_t& e : g_res.ev) NRPYELL_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   }
   if (g_res.bytes < bytes) {
@@ -1209,7 +1209,7 @@ bool relax_resident(const std::vector<ResGrid>& grids, std::vector<RelaxResult>*
     NRPYELL_CUDA(cudaMemcpy(&st[4 * i], grids[i].state, sizeof(int) * 4, cudaMemcpyDeviceToHost));
   NRPYELL_CUDA(cudaMemcpy(&err, g_res.err, sizeof(int), cudaMemcpyDeviceToHost));
   if (err) {
-    NRPYELL_CUDA(cudaMemset(g_res.err, 0, sizeof(int)));
+    NRPYELL_CUDA(cudaMemsetAsync(g_res.err, 0, sizeof(int), stream()));
     NRPYELL_FAIL("on-chip relaxation: a bounded wait for a neighbouring block gave up");
   }
   if (!status_ok()) return false;

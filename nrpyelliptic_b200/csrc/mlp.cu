@@ -343,7 +343,7 @@ void launch_products(GemmArgs& g) {
   }
   if (!g_tc_err) {
     NRPYELL_CUDA(dev_alloc(&g_tc_err, sizeof(int)));
-    NRPYELL_CUDA(cudaMemset(g_tc_err, 0, sizeof(int)));
+    NRPYELL_CUDA(cudaMemsetAsync(g_tc_err, 0, sizeof(int), stream()));
   }
   int blocks = (g.cs_cols + 127) / 128;
   for (Product& p : g.p) {
@@ -366,7 +366,7 @@ bool gemm_ok() {
   int e = 0;
   NRPYELL_CUDA(cudaMemcpy(&e, g_tc_err, sizeof(int), cudaMemcpyDeviceToHost));
   if (e) {
-    NRPYELL_CUDA(cudaMemset(g_tc_err, 0, sizeof(int)));
+    NRPYELL_CUDA(cudaMemsetAsync(g_tc_err, 0, sizeof(int), stream()));
     NRPYELL_FAIL("k_gemm_tc: a bounded wait for the tensor-core products gave up");
     return false;
   }

@@ -26,8 +26,12 @@ void* table_alloc(size_t bytes) {
   return p;
 }
 
+// On the library's stream: a plain copy from pageable memory may still be on its
+// way when it returns, and that stream does not wait for the default stream.
 void upload(void* dst, const void* src, size_t bytes) {
-  if (bytes) NRPYELL_CUDA(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice));
+  if (!bytes) return;
+  NRPYELL_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream()));
+  NRPYELL_CUDA(cudaStreamSynchronize(stream()));
 }
 
 }  // namespace
@@ -352,7 +356,7 @@ Scratch* get_scratch(int n_partials) {
   s->n_partials = n_partials < 4096 ? 4096 : n_partials;
   const size_t bytes = (size_t)s->n_partials * 8 + 4 * 8 + 64 + 8 * 4 + 256;
   char* base = (char*)table_alloc(bytes);
-  NRPYELL_CUDA(cudaMemset(base, 0, bytes));
+  NRPYELL_CUDA(cudaMemsetAsync(base, 0, bytes, stream()));
   s->base = base;
   s->partials = (double*)base;
   s->result = (double*)(base + (size_t)s->n_partials * 8);
