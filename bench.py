@@ -464,8 +464,10 @@ def run_ours(args, dist):
     lib.nrpyell_host_pinned_free(aux_h)
     lib.nrpyell_host_pinned_free(y_h)
 
-    # Roofline of the dominant kernel: the fused RK4 substep (RHS + radiation
-    # BC + RK combination), stage 2, timed over 200 graph-replayed launches.
+    # Roofline of the fused RK4 substep (RHS + radiation BC + RK combination),
+    # which steps grids that do not fit on chip: stage 2, timed over 200
+    # graph-replayed launches.  The timed solves above run on chip
+    # (k_relax_resident), where only block edges leave the SMs.
     peak, peak_kind = measured_hbm_peak()
     n_int = cfg.Nxx[0] * cfg.Nxx[1] * cfg.Nxx[2]
     ms_k, ms_s = C.c_double(0), C.c_double(0)

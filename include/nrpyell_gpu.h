@@ -139,7 +139,8 @@ void nrpyell_set_async(int enable);
  * stepped and keeps the fastest.  nrpyell_set_tile(t) forces shape t, for
  * every grid (-1: the default);
  * nrpyell_get_tile reports the shape in use for a grid (block 32 x by threads,
- * `planes` consecutive i2 planes per thread), -1 if not tuned yet; its fp32
+ * `planes` consecutive i2 planes per thread), -1 if none was timed yet (a grid
+ * that only relaxed on chip); its fp32
  * argument selects FP64 (0), FP32 (1) or the FP32 correction form of
  * nrpyell_relax_mixed (2: marching shapes and the 8-warp direct shapes).
  * nrpyell_num_tiles gives the number of shapes; nrpyell_tile_info describes
