@@ -936,48 +936,52 @@ ResKernel<T> resident_kernel(int tx, int p) {
   return nullptr;
 }
 
+// Device memory that only grows.
+struct ResidentArea {
+  size_t bytes = 0;
+  unsigned char* mem = nullptr;
+};
+
 // Work memory of the on-chip driver, kept between calls until
-// nrpyell_release_tables.
+// nrpyell_release_tables.  Values are told from older ones by their tags alone,
+// so a word that is read as a tag must never have held anything else since it
+// was cleared: the exchange slots of FP64 (value and tag in 16 bytes), those of
+// FP32 (8 bytes) and the residual shares have an area each, in which every
+// layout has its tags at the same places.
 struct ResidentWork {
-  size_t bytes = 0, jobs_bytes = 0;
-  unsigned char* mem = nullptr;   // exchange slots and residual shares
-  unsigned char* jobs = nullptr;
+  ResidentArea slots[2], shares;  // slots: FP64, FP32
+  ResidentArea jobs;
   int* err = nullptr;
   int* pinned = nullptr;          // polled states of two launches
   size_t pinned_ints = 0;
   cudaEvent_t ev[2] = {nullptr, nullptr};
-  unsigned version = 0;           // last tag used in mem
+  unsigned version = 0;           // last tag used in slots and shares
 };
 ResidentWork g_res;
 
 size_t align_up(size_t n) { return (n + 255) / 256 * 256; }
 
-bool ensure_resident(size_t bytes, size_t jobs_bytes, size_t pinned_ints) {
+bool grow(ResidentArea* a, size_t bytes) {
+  if (a->bytes >= bytes) return true;
+  NRPYELL_CUDA(cudaStreamSynchronize(stream()));
+  cudaFree(a->mem);
+  *a = ResidentArea();
+  NRPYELL_CUDA(dev_alloc(&a->mem, bytes));
+  if (!status_ok()) return false;
+  NRPYELL_CUDA(cudaMemsetAsync(a->mem, 0, bytes, stream()));
+  a->bytes = bytes;
+  return status_ok();
+}
+
+bool ensure_resident(bool fp64, size_t slot_bytes, size_t share_bytes, size_t jobs_bytes, size_t pinned_ints) {
   if (!g_res.err) {
     NRPYELL_CUDA(dev_alloc(&g_res.err, sizeof(int)));
     NRPYELL_CUDA(cudaMemsetAsync(g_res.err, 0, sizeof(int), stream()));
     for (cudaEvent_t& e : g_res.ev) NRPYELL_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   }
-  if (g_res.bytes < bytes) {
-    NRPYELL_CUDA(cudaStreamSynchronize(stream()));
-    cudaFree(g_res.mem);
-    g_res.mem = nullptr;
-    g_res.bytes = 0;
-    NRPYELL_CUDA(dev_alloc(&g_res.mem, bytes));
-    if (!status_ok()) return false;
-    NRPYELL_CUDA(cudaMemsetAsync(g_res.mem, 0, bytes, stream()));
-    g_res.bytes = bytes;
-    g_res.version = 0;
-  }
-  if (g_res.jobs_bytes < jobs_bytes) {
-    NRPYELL_CUDA(cudaStreamSynchronize(stream()));
-    cudaFree(g_res.jobs);
-    g_res.jobs = nullptr;
-    g_res.jobs_bytes = 0;
-    NRPYELL_CUDA(dev_alloc(&g_res.jobs, jobs_bytes));
-    if (!status_ok()) return false;
-    g_res.jobs_bytes = jobs_bytes;
-  }
+  if (!grow(&g_res.slots[fp64 ? 0 : 1], slot_bytes) || !grow(&g_res.shares, share_bytes) ||
+      !grow(&g_res.jobs, jobs_bytes))
+    return false;
   if (g_res.pinned_ints < pinned_ints) {
     NRPYELL_CUDA(cudaStreamSynchronize(stream()));
     cudaFreeHost(g_res.pinned);
@@ -998,8 +1002,7 @@ constexpr int kStepsPerLaunch = 512;
 }  // namespace
 
 void release_resident() {
-  cudaFree(g_res.mem);
-  cudaFree(g_res.jobs);
+  for (ResidentArea* a : {&g_res.slots[0], &g_res.slots[1], &g_res.shares, &g_res.jobs}) cudaFree(a->mem);
   cudaFree(g_res.err);
   cudaFreeHost(g_res.pinned);
   for (cudaEvent_t e : g_res.ev)
@@ -1087,8 +1090,8 @@ bool relax_resident(const std::vector<ResGrid>& grids, std::vector<RelaxResult>*
   const int n = (int)grids.size();
   const int sms = device_attr(cudaDevAttrMultiProcessorCount);
   std::vector<ResJob<T>> jobs(n);
-  size_t bytes = 0;
-  std::vector<size_t> off(2 * n);
+  size_t slot_bytes = 0, share_bytes = 0;
+  std::vector<size_t> slot_off(n), share_off(n);
   ResPlan plan = resident_plan<T>(grids[0].d, sms / n);
   if (plan.blocks == 0) {
     NRPYELL_FAIL("relax_resident: the grid does not fit");
@@ -1126,10 +1129,10 @@ bool relax_resident(const std::vector<ResGrid>& grids, std::vector<RelaxResult>*
     J.xv_plane = d.Nxx1 * 12;
     J.xv0 = J.xu_plane * d.Nxx2;
     J.xu_slot = (long long)J.xv0 + J.xv_plane * d.Nxx2;
-    off[2 * i] = bytes;
-    bytes += align_up(sizeof(Raw) * kSlots * J.xu_slot);
-    off[2 * i + 1] = bytes;
-    bytes += align_up(sizeof(double2) * 2 * J.n0t * J.n1t);
+    slot_off[i] = slot_bytes;
+    slot_bytes += align_up(sizeof(Raw) * kSlots * J.xu_slot);
+    share_off[i] = share_bytes;
+    share_bytes += align_up(sizeof(double2) * 2 * J.n0t * J.n1t);
     J.state = g.state;
     J.sums = g.history;
     J.volume = g.lt->volume;
@@ -1157,18 +1160,19 @@ bool relax_resident(const std::vector<ResGrid>& grids, std::vector<RelaxResult>*
     max_steps = std::max(max_steps, g.rp.max_steps);
   }
   const int stride = 4 * n;  // ints per polled launch
-  if (!ensure_resident(bytes, sizeof(ResJob<T>) * n, 2 * (stride + 1))) return false;
+  constexpr bool fp64 = sizeof(T) == 8;
+  if (!ensure_resident(fp64, slot_bytes, share_bytes, sizeof(ResJob<T>) * n, 2 * (stride + 1))) return false;
   for (int i = 0; i < n; i++) {
-    jobs[i].xu = g_res.mem + off[2 * i];
-    jobs[i].part = (double2*)(g_res.mem + off[2 * i + 1]);
+    jobs[i].xu = g_res.slots[fp64 ? 0 : 1].mem + slot_off[i];
+    jobs[i].part = (double2*)(g_res.shares.mem + share_off[i]);
     jobs[i].err = g_res.err;
     NRPYELL_CUDA(cudaMemsetAsync(grids[i].state, 0, sizeof(int) * 4, stream()));
   }
-  NRPYELL_CUDA(cudaMemcpyAsync(g_res.jobs, jobs.data(), sizeof(ResJob<T>) * n, cudaMemcpyHostToDevice, stream()));
+  NRPYELL_CUDA(cudaMemcpyAsync(g_res.jobs.mem, jobs.data(), sizeof(ResJob<T>) * n, cudaMemcpyHostToDevice, stream()));
   ResKernel<T> kern = resident_kernel<T>(plan.tx, plan.p);
   NRPYELL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem));
   if (!status_ok()) return false;
-  const ResJob<T>* jobs_dev = (const ResJob<T>*)g_res.jobs;
+  const ResJob<T>* jobs_dev = (const ResJob<T>*)g_res.jobs.mem;
   int njobs = n;
   // max_steps + 1 residuals are evaluated at most; the states of a launch are
   // read while the next one runs
@@ -1177,7 +1181,8 @@ bool relax_resident(const std::vector<ResGrid>& grids, std::vector<RelaxResult>*
     int steps = (int)std::min<long long>(kStepsPerLaunch, left);
     left -= steps;
     if (g_res.version > 0xf0000000u) {  // tags are about to wrap: start again from cleared slots
-      NRPYELL_CUDA(cudaMemsetAsync(g_res.mem, 0, g_res.bytes, stream()));
+      for (const ResidentArea* a : {&g_res.slots[0], &g_res.slots[1], &g_res.shares})
+        if (a->bytes) NRPYELL_CUDA(cudaMemsetAsync(a->mem, 0, a->bytes, stream()));
       g_res.version = 0;
     }
     unsigned base = g_res.version;
