@@ -273,7 +273,7 @@ __device__ __forceinline__ int stop_test(const ResJob<T>& J, int local, int n, u
       J.sums[n] = s;
       if (met) J.state[2] = 1;
       if (stop)
-        J.state[1] = 1;
+        J.state[1] = stop_mark(n);
       else
         J.state[0] = n + 1;
     }
@@ -873,27 +873,25 @@ __device__ __forceinline__ void radiation_block(const ResJob<T>& J, int local, u
   }
 }
 
-// Up to `steps` RK4 steps of every job; block b belongs to the last job with
-// cta0 <= b.  Exchanged values of this launch carry tags base + 1 ..
+// Up to `steps` RK4 steps of every job from step `first` on; block b belongs to
+// the last job with cta0 <= b.  Exchanged values of this launch carry tags base + 1 ..
 // base + 4 steps.
 template <typename T, bool CORR, int TX, int P2>
 __global__ void __launch_bounds__(kThreads, 1)
-    k_relax_resident(const ResJob<T>* __restrict__ jobs, int njobs, unsigned base, int steps) {
+    k_relax_resident(const ResJob<T>* __restrict__ jobs, int njobs, unsigned base, int steps, int first) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ BlockState bs;
   __shared__ ResJob<T> J;
   int j = 0;
   while (j + 1 < njobs && (int)blockIdx.x >= jobs[j + 1].cta0) j++;
-  // the job's first block advances state[0] only after every block of the
-  // job has published a value, so all blocks read the same state here
   if (threadIdx.x == 0) {
     J = jobs[j];
-    J.n_start = J.state[0];
-    bs.stop = J.state[1];
+    J.n_start = first;
+    bs.stop = stopped_before(*(volatile int*)(J.state + 1), first);
     bs.failed = 0;
   }
   __syncthreads();
-  if (bs.stop) return;  // done before this launch
+  if (bs.stop) return;
   const int local = (int)blockIdx.x - J.cta0;
   if (local < J.n0t * J.n1t)
     interior_block<T, CORR, TX, P2>(J, local, base, steps, smem, &bs);
@@ -923,7 +921,7 @@ constexpr int kTX[] = {8, 16};
 constexpr int kP[] = {1, 2, 3};  // planes of a thread per half
 
 template <typename T>
-using ResKernel = void (*)(const ResJob<T>*, int, unsigned, int);
+using ResKernel = void (*)(const ResJob<T>*, int, unsigned, int, int);
 
 template <typename T>
 ResKernel<T> resident_kernel(int tx, int p) {
@@ -1178,7 +1176,7 @@ bool relax_resident(const std::vector<ResGrid>& grids, std::vector<RelaxResult>*
   // read while the next one runs
   long long left = (long long)max_steps + 1;
   for (long long k = 0; left > 0; k++) {
-    int steps = (int)std::min<long long>(kStepsPerLaunch, left);
+    int steps = (int)std::min<long long>(kStepsPerLaunch, left), first = (int)(kStepsPerLaunch * k);
     left -= steps;
     if (g_res.version > 0xf0000000u) {  // tags are about to wrap: start again from cleared slots
       for (const ResidentArea* a : {&g_res.slots[0], &g_res.slots[1], &g_res.shares})
@@ -1187,7 +1185,7 @@ bool relax_resident(const std::vector<ResGrid>& grids, std::vector<RelaxResult>*
     }
     unsigned base = g_res.version;
     g_res.version += 4 * steps;
-    void* args[] = {(void*)&jobs_dev, (void*)&njobs, (void*)&base, (void*)&steps};
+    void* args[] = {(void*)&jobs_dev, (void*)&njobs, (void*)&base, (void*)&steps, (void*)&first};
     NRPYELL_CUDA(cudaLaunchCooperativeKernel((const void*)kern, dim3(blocks), dim3(plan.threads), args, plan.smem,
                                              stream()));
     count_launch();

@@ -29,7 +29,7 @@ struct ResJob {
   long long xu_slot;             // entries of a slot: uu, then vv from xv0 on
   int xu_row, xu_plane, xv0, xv_plane;
   double2* part;                 // [2][interior blocks]: shares of the residual norm
-  int* state;                    // [0] n, [1] done, [2] converged
+  int* state;                    // [0] n, [1] 0 or the stop mark, [2] converged
   double* sums;                  // weighted sum of squares of every evaluated residual
   int* err;
   double volume, log10_tol;
@@ -40,6 +40,14 @@ struct ResJob {
   double invdx0, invdx1;
   int n_start;                   // filled in by the kernel
 };
+
+// The stop mark of a job that ended at step n.  Blocks read it as they start, and
+// block 0 may write it meanwhile (nothing orders its first stop test after the
+// start of a radiation block), so a mark made by the launch itself must read
+// as none: with the launch's first step, passed by the host, both values mean
+// the same to every block.
+__host__ __device__ inline int stop_mark(int n) { return n + 1; }
+__host__ __device__ inline bool stopped_before(int mark, int first) { return mark != 0 && mark <= first; }
 
 // One grid to relax on chip.
 struct ResGrid {

@@ -105,9 +105,56 @@ void relax(const std::vector<FakeGrid*>& grids) {
   if (!relax_resident<T>(gs, &r)) g_faults++;
 }
 
+// A launch as the jobs' block 0 leaves it, for jobs that end at g_stop[j]: what
+// any other block makes of the state must not depend on when it reads it.
+std::vector<int> g_stop;
+int g_next_first = 0;
+void on_stepping_launch(const void*, dim3, dim3, void** args, size_t) {
+  const ResJob<double>* jobs = *(const ResJob<double>**)args[0];
+  const int njobs = *(int*)args[1], steps = *(int*)args[3], first = *(int*)args[4];
+  if (first != g_next_first) g_faults++;
+  g_next_first = first + steps;
+  for (int j = 0; j < njobs; j++) {
+    int* st = jobs[j].state;
+    const bool over = stopped_before(st[1], first);
+    if (over != (g_stop[j] < first)) g_faults++;
+    for (int n = first; !over && n < first + steps; n++) {
+      if (n == g_stop[j])
+        st[1] = stop_mark(n);
+      else
+        st[0] = n + 1;
+      if (stopped_before(st[1], first)) g_faults++;
+      if (n == g_stop[j]) break;
+    }
+  }
+}
+
 }  // namespace
 
 extern "C" {
+
+// Jobs that end at the given steps of several launches.
+int check_start_state(const int* stop, int n) {
+  g_faults = 0;
+  g_next_first = 0;
+  g_stop.assign(stop, stop + n);
+  std::vector<FakeGrid*> grids;
+  std::vector<ResGrid> gs;
+  for (int j = 0; j < n; j++) {
+    grids.push_back(new FakeGrid(24, 17, 8, -10.0, 1600, 1.0));
+    gs.push_back(grids[j]->g);
+  }
+  std::vector<RelaxResult> r;
+  g_fake_cooperative = on_stepping_launch;
+  if (!relax_resident<double>(gs, &r)) g_faults++;
+  g_fake_cooperative = nullptr;
+  for (int j = 0; j < n; j++) {
+    if (r[j].steps != stop[j]) g_faults++;
+    delete grids[j];
+  }
+  release_resident();
+  return g_faults;
+}
 
 // FP64 and FP32 launches in turn, of several grids and team sizes: no word that
 // one of them reads as a tag may hold what another wrote as a value.
