@@ -260,13 +260,7 @@ __device__ __forceinline__ int stop_test(const ResJob<T>& J, int local, int n, u
   if (lane == 0) {
     bool test = true;
     if (J.check_every > 0) test = n >= 1 && ((n - 1) % J.check_every == 0 || n >= J.max_steps);
-    // far from the tolerance the sum itself decides; log10 only near it
-    bool met = s <= J.sum_met;
-    if (!met && !(s >= J.sum_not_met)) {
-      const double l2 = log10(1e-16 + sqrt(s / J.volume));
-      met = J.check_every > 0 ? l2 < J.log10_tol : l2 <= J.log10_tol;
-    }
-    met = met && test;
+    const bool met = test && residual_met(J, s);
     const bool stop = met || n >= J.max_steps;
     bs->stop = stop;
     if (local == 0 && ok) {
@@ -1136,14 +1130,17 @@ bool relax_resident(const std::vector<ResGrid>& grids, std::vector<RelaxResult>*
     J.volume = g.lt->volume;
     J.log10_tol = g.rp.log10_tol;
     // log10(1e-16 + sqrt(s / volume)) against the tolerance: decided by the
-    // sum alone more than 1e-9 away from it
-    const double t = g.rp.log10_tol;
-    J.sum_met = -1.0;
-    J.sum_not_met = INFINITY;
+    // sum alone more than 1e-9 away from it.  Not where the volume is 0 (no
+    // point within the integration radius: the norm is NaN and never meets a
+    // tolerance) or the sum at the tolerance is no normal number.
+    const double t = g.rp.log10_tol, vol = g.lt->volume;
+    J.sum_met = J.sum_not_met = NAN;
     if (t > -15.0) {
-      const double root = pow(10.0, t) - 1e-16;
-      J.sum_met = g.lt->volume * root * root * (1.0 - 1e-9);
-      J.sum_not_met = g.lt->volume * root * root * (1.0 + 1e-9);
+      const double root = pow(10.0, t) - 1e-16, at = vol * root * root;
+      if (at > 1e-300 && at < 1e300) {
+        J.sum_met = at * (1.0 - 1e-9);
+        J.sum_not_met = at * (1.0 + 1e-9);
+      }
     } else if (t < -17.0) {
       J.sum_not_met = 0.0;
     }

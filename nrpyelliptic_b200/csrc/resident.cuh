@@ -2,6 +2,8 @@
 // and the host driver's interface.
 #pragma once
 
+#include <math.h>
+
 #include <vector>
 
 #include "driver.cuh"
@@ -33,7 +35,7 @@ struct ResJob {
   double* sums;                  // weighted sum of squares of every evaluated residual
   int* err;
   double volume, log10_tol;
-  double sum_met, sum_not_met;   // sums at or below / above which the stop test needs no logarithm
+  double sum_met, sum_not_met;   // sums at or below / above which the stop test needs no logarithm (NaN: none)
   int max_steps, check_every;
   T dt, eta;
   T cOB[2];
@@ -48,6 +50,16 @@ struct ResJob {
 // the same to every block.
 __host__ __device__ inline int stop_mark(int n) { return n + 1; }
 __host__ __device__ inline bool stopped_before(int mark, int first) { return mark != 0 && mark <= first; }
+
+// Whether a weighted sum of squares meets the tolerance: finalize_l2's test,
+// without its logarithm where the sum alone decides.
+template <typename Job>
+__host__ __device__ inline bool residual_met(const Job& J, double s) {
+  if (s <= J.sum_met) return true;
+  if (s >= J.sum_not_met) return false;
+  const double l2 = log10(1e-16 + sqrt(s / J.volume));
+  return J.check_every > 0 ? l2 < J.log10_tol : l2 <= J.log10_tol;
+}
 
 // One grid to relax on chip.
 struct ResGrid {

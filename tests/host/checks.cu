@@ -129,9 +129,34 @@ void on_stepping_launch(const void*, dim3, dim3, void** args, size_t) {
   }
 }
 
+// The stop test of a launch's job against the plain rule (finalize_l2).
+std::vector<double> g_sums;
+void on_launch_compare_stop(const void*, dim3, dim3, void** args, size_t) {
+  const ResJob<double>& J = **(const ResJob<double>**)args[0];
+  for (double s : g_sums) {
+    const double l2 = log10(1e-16 + sqrt(s / J.volume));
+    if (residual_met(J, s) != (J.check_every > 0 ? l2 < J.log10_tol : l2 <= J.log10_tol)) {
+      g_faults++;
+      fprintf(stderr, "sum %g, volume %g, tolerance %g\n", s, J.volume, J.log10_tol);
+    }
+  }
+}
+
 }  // namespace
 
 extern "C" {
+
+int check_stop_rule(double log10_tol, double volume, int check_every, const double* sums, int n) {
+  g_faults = 0;
+  g_sums.assign(sums, sums + n);
+  FakeGrid a(24, 17, 8, log10_tol, 0, volume);
+  a.g.rp.check_every = check_every;
+  g_fake_cooperative = on_launch_compare_stop;
+  relax<double>({&a});
+  g_fake_cooperative = nullptr;
+  release_resident();
+  return g_faults;
+}
 
 // Jobs that end at the given steps of several launches.
 int check_start_state(const int* stop, int n) {
