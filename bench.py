@@ -193,47 +193,28 @@ def cpu_time_per_iteration(cfg, seconds, threads=None):
     return t_done / n_done, kind, cores, n_done
 
 
-def cpu_solver(cfg):
+def cpu_solver(cfg, ref):
     """One complete solve of cfg from the zero guess on the host cores per
-    call: the reference's own build (main.c's loop with the stop test,
-    refh_relax) when present, else the oracle port.  Returns (solve,
-    cleanup, kind, cores); solve() returns (seconds, steps, converged)."""
+    call, by the reference's own build `ref` (main.c's loop with the stop test,
+    refh_relax).  Returns (solve, cleanup, cores); solve() returns (seconds,
+    steps, converged)."""
     from nrpyelliptic_b200 import abi
     from nrpyelliptic_b200.problem import set_physical_params
-    from oracle import build as obuild
-    ref = obuild.ref_lib_path(cpu_isa())
     P = C.POINTER
-    if os.path.exists(ref):
-        lib = C.CDLL(ref)
-        lib.refh_setup.restype = C.c_double
-        lib.refh_setup.argtypes = [P(abi.griddata_struct), P(C.c_int), P(abi.paramstruct), C.c_double]
-        lib.refh_relax.restype = C.c_int
-        lib.refh_relax.argtypes = [P(abi.griddata_struct), C.c_double, C.c_double, C.c_int, C.c_double, abi.PREAL,
-                                   P(C.c_int)]
-        lib.refh_free.argtypes = [P(abi.griddata_struct)]
-        lib.refh_max_threads.restype = C.c_int
-        lib.set_Cparameters_to_default.argtypes = [P(abi.paramstruct)]
-        phys = abi.paramstruct()
-        lib.set_Cparameters_to_default(C.byref(phys))
-        set_physical_params(phys, cfg)
-        g = abi.griddata_struct()
-        dt = lib.refh_setup(C.byref(g), (C.c_int * 3)(*cfg.Nxx), C.byref(phys), cfg.CFL)
-        relax = lib.refh_relax
-        kind, cores = "reference", lib.refh_max_threads()
-        cleanup = lambda: lib.refh_free(C.byref(g))
-    else:
-        sys.path.insert(0, os.path.join(ROOT, "tests"))
-        from _util import oracle, problem_grid
-
-        from nrpyelliptic_b200.problem import Problem
-        o = oracle()
-        prob = Problem(cfg)
-        hg = problem_grid(prob)
-        g = hg.griddata()
-        dt = prob.dt
-        relax = o.oracle_relax
-        kind, cores = "port", os.cpu_count()
-        cleanup = lambda: None
+    lib = C.CDLL(ref)
+    lib.refh_setup.restype = C.c_double
+    lib.refh_setup.argtypes = [P(abi.griddata_struct), P(C.c_int), P(abi.paramstruct), C.c_double]
+    lib.refh_relax.restype = C.c_int
+    lib.refh_relax.argtypes = [P(abi.griddata_struct), C.c_double, C.c_double, C.c_int, C.c_double, abi.PREAL,
+                               P(C.c_int)]
+    lib.refh_free.argtypes = [P(abi.griddata_struct)]
+    lib.refh_max_threads.restype = C.c_int
+    lib.set_Cparameters_to_default.argtypes = [P(abi.paramstruct)]
+    phys = abi.paramstruct()
+    lib.set_Cparameters_to_default(C.byref(phys))
+    set_physical_params(phys, cfg)
+    g = abi.griddata_struct()
+    dt = lib.refh_setup(C.byref(g), (C.c_int * 3)(*cfg.Nxx), C.byref(phys), cfg.CFL)
     p = g.params
     n2 = 2 * p.Nxx_plus_2NGHOSTS0 * p.Nxx_plus_2NGHOSTS1 * p.Nxx_plus_2NGHOSTS2 * 8
 
@@ -241,21 +222,27 @@ def cpu_solver(cfg):
         C.memset(g.gridfuncs.y_n_gfs, 0, n2)  # initial_guess_all_points: uu = vv = 0
         steps = C.c_int(0)
         t0 = time.perf_counter()
-        rc = relax(C.byref(g), dt, TOL, max_steps, cfg.R_L2, None, C.byref(steps))
+        rc = lib.refh_relax(C.byref(g), dt, TOL, max_steps, cfg.R_L2, None, C.byref(steps))
         return time.perf_counter() - t0, steps.value, rc == 0
 
-    return solve, cleanup, kind, cores
+    return solve, lambda: lib.refh_free(C.byref(g)), lib.refh_max_threads()
 
 
 def run_reference(args, dist):
     """The reference's own CPU implementation of the path: every bench step is
     one complete solve of the workload from the zero guess to the tolerance
-    (main.c's loop: residual, L2, RK4 step, with the stop test)."""
+    (main.c's loop: residual, L2, RK4 step, with the stop test).  Without the
+    reference's build there is nothing to measure, and the line says so."""
     from nrpyelliptic_b200.problem import CONFIGS
+    from oracle import build as obuild
     if dist.rank != 0:
         return
+    ref = obuild.ref_lib_path(cpu_isa())
+    if not os.path.exists(ref):
+        print(json.dumps({"impl": "reference", "unavailable": "no build of the reference's sources in oracle/_ref"}))
+        return
     cfg = CONFIGS[args.config]
-    solve, cleanup, kind, cores = cpu_solver(cfg)
+    solve, cleanup, cores = cpu_solver(cfg, ref)
     times, steps_seen = [], set()
     for i in range(args.warmup + args.steps):
         t, n, ok = solve(args.max_steps)
@@ -277,7 +264,7 @@ def run_reference(args, dist):
             "impl": "reference",
             "config": {"workload": args.config, "grid": list(cfg.Nxx), "tolerance_log10": TOL,
                        "steps_to_tolerance": max(steps_seen), "parallelism": "host OpenMP"},
-            "cpu_baseline": {"value": value, "unit": "solves/s", "cores": cores, "kind": kind, "sample": sample},
+            "cpu_baseline": {"value": value, "unit": "solves/s", "cores": cores, "kind": "reference", "sample": sample},
             "e2e": {"value": value, "unit": "solves/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
             "per_iteration_sample": {"s_per_iteration": t_it, "iterations": n_it,
                                      "solves_per_s_extrapolated": 1.0 / (t_it * (max(steps_seen) + 1))}}
