@@ -290,16 +290,15 @@ __global__ void __launch_bounds__(TC_THREADS) k_gemm_tc(const __grid_constant__ 
       for (int j = 0; j < 8; j++)
         if (j < cols) P.out[at + j] = f[j];
     }
-    if (P.row) {
-      bf16* const o = P.row + (long long)m * P.ld_row + nc;
-      if (cols == 8) {
-        *reinterpret_cast<uint4*>(o) =
-            make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
-      } else {
+    // a row is zero from N to the next multiple of 16: the product that reads it
+    // sums up to there, and the same memory may have held longer rows (zero
+    // weights would not cancel infinities or NaNs of an earlier pass)
+    if (P.row && live && nc < (N + 15) / 16 * 16) {
 #pragma unroll
-        for (int j = 0; j < 8; j++)
-          if (j < cols) o[j] = __float2bfloat16_rn(f[j]);
-      }
+      for (int j = 0; j < 8; j++)
+        if (j >= cols) f[j] = 0.f;
+      *reinterpret_cast<uint4*>(P.row + (long long)m * P.ld_row + nc) =
+          make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
     }
     if (P.col && m < mpad) {
       bf16* o = P.col + (long long)nc * P.ld_col + m;
@@ -481,7 +480,9 @@ struct Mlp {
   std::vector<float*> h;   // output of layer l [batch_max x dims[l+1]]
   float* t = nullptr;      // minibatch targets
   float* dz[2] = {nullptr, nullptr};  // dZ of two consecutive layers [batch_max x widest]
-  // BF16 operands, leading dimensions a multiple of 64 and zero padding:
+  // BF16 operands, leading dimensions a multiple of 64 and zero padding up to the
+  // next multiple of 16 (the epilogue writes it: dZ's memory serves layers of
+  // several lengths):
   // hb[l] the input of layer l [batch_max x dims[l]] and its transpose, wb[l]
   // W_l and its transpose, db / dbt dZ of two consecutive layers
   std::vector<bf16*> hb, hbt, wb, wbt;
