@@ -853,7 +853,10 @@ double nrpyell_mlp_train(void* mlp, const float* x, const float* t, int n, int b
     if (!status_ok()) return NAN;
     q->idx_cap = n;
   }
-  std::vector<int> perm(n);
+  // perm is shuffled while the previous epoch runs; the copy to the GPU reads
+  // `order`, which changes only after a wait for the epoch that it belongs to (an
+  // asynchronous copy may read pageable memory at any time until then)
+  std::vector<int> perm(n), order(n);
   for (int i = 0; i < n; i++) perm[i] = i;
   unsigned long long s = 0xD1B54A32D192ED03ull ^ seed;
   const int per_epoch = n / batch;
@@ -861,8 +864,6 @@ double nrpyell_mlp_train(void* mlp, const float* x, const float* t, int n, int b
   long long it = 0;
   double last = NAN;
   for (int e = 0; e < epochs && status_ok(); e++) {
-    // shuffled while the previous epoch runs (its index copy was taken at the
-    // call: pageable memory)
     for (int i = n - 1; i > 0; i--) {  // Fisher-Yates
       s = s * 6364136223846793005ull + 1442695040888963407ull;
       const int j = (int)((s >> 33) % (unsigned long long)(i + 1));
@@ -879,7 +880,8 @@ double nrpyell_mlp_train(void* mlp, const float* x, const float* t, int n, int b
       if (loss_history) loss_history[e - 1] = last;
     }
     NRPYELL_CUDA(cudaMemsetAsync(q->loss, 0, sizeof(double), stream()));
-    NRPYELL_CUDA(cudaMemcpyAsync(q->idx, perm.data(), sizeof(int) * n, cudaMemcpyHostToDevice, stream()));
+    order = perm;
+    NRPYELL_CUDA(cudaMemcpyAsync(q->idx, order.data(), sizeof(int) * n, cudaMemcpyHostToDevice, stream()));
     for (int b = 0; b < per_epoch; b++, it++) {
       mlp_inputs(q, x, t, q->idx + (long long)b * batch, batch);
       mlp_forward(q, batch, true);

@@ -32,3 +32,31 @@ def test_stop_test_follows_the_plain_rule(lib, tol, volume, check_every):
                     + [near * f for f in (0.5, 1 - 1e-6, 1 - 1e-8, 1 + 1e-8, 1 + 1e-6, 2.0)])
     assert lib.check_stop_rule(C.c_double(tol), C.c_double(volume), check_every,
                                sums.ctypes.data_as(C.POINTER(C.c_double)), len(sums)) == 0
+
+
+def test_training_order_is_not_reshuffled_under_its_copy(lib):
+    """Every epoch's row order reaches the GPU as it was drawn: the memory it is
+    copied from stays as it is until the copy has happened."""
+    n, epochs, seed = 83, 5, 7
+    lib.nrpyell_mlp_create.restype = C.c_void_p
+    lib.nrpyell_mlp_train.restype = C.c_double
+    lib.fake_logged.restype = C.c_size_t
+    q = C.c_void_p(lib.nrpyell_mlp_create(13, 32, 2, 8, 16, 3))
+    rows = np.zeros((n, 13), np.float32)
+    lib.fake_log_copies(C.c_size_t(4 * n))
+    lib.nrpyell_mlp_train(q, rows.ctypes.data_as(C.c_void_p), rows.ctypes.data_as(C.c_void_p), n, 16, epochs,
+                          C.c_float(1e-3), seed, None)
+    got = np.zeros(2 * epochs * n, np.int32)
+    used = lib.fake_logged(got.ctypes.data_as(C.c_void_p), C.c_size_t(got.nbytes))
+    lib.fake_log_copies(C.c_size_t(0))
+    lib.nrpyell_mlp_destroy(q)
+    mask = (1 << 64) - 1
+    s, perm, want = 0xD1B54A32D192ED03 ^ seed, list(range(n)), []
+    for _ in range(epochs):
+        for i in range(n - 1, 0, -1):
+            s = (s * 6364136223846793005 + 1442695040888963407) & mask
+            j = (s >> 33) % (i + 1)
+            perm[i], perm[j] = perm[j], perm[i]
+        want.append(list(perm))
+    assert used == 4 * epochs * n
+    np.testing.assert_array_equal(got[:epochs * n].reshape(epochs, n), want)
