@@ -105,6 +105,8 @@ bool build_devs(const std::vector<Grid>& grids, int tile, std::vector<SubDev<T>>
   devs->assign(5 * n, SubDev<T>());
   offs->assign(n, 0);
   int total = 0;
+  double points = 0.0;
+  for (const Grid& g : grids) points += (double)g.d.Ntot;
   for (int c = 0; c < n; c++) {
     const Grid& g = grids[c];
     Scratch sc;
@@ -123,6 +125,7 @@ bool build_devs(const std::vector<Grid>& grids, int tile, std::vector<SubDev<T>>
         a.max_steps = g.rp.max_steps;
       }
       if (!batch_launch_dev<T>(a, &(*devs)[k * n + c])) return false;
+      (*devs)[k * n + c].alternate = march_alternates<T>(points, g.b.R0 != nullptr);
     }
     const SubDev<T>& f = (*devs)[c];
     if (f.n_tiles > g_batch.partials_per) {

@@ -68,11 +68,11 @@ struct MarchSmem {
   static constexpr size_t bytes = march > cols ? march : cols;
 };
 
-// Whether a substep sweeps its planes (and, in a batch, its grids) from the
-// last to the first.  A substep touches 11 fields, more than L2 holds from
-// 256x256x32 on, and blocks run in index order, so sweeping every substep the
-// same way evicts each plane before the next substep comes to it.
-__device__ constexpr bool march_reversed(int stage) { return stage == 2 || stage == 4; }
+// Whether this substep sweeps from the last plane (and grid) to the first.
+template <typename T, int STAGE>
+__device__ __forceinline__ bool march_reversed(const SubDev<T>& a) {
+  return (STAGE == 2 || STAGE == 4) && a.alternate;
+}
 
 // Block `bid` of one grid's marching launch; dsm is the block's dynamic
 // shared memory (MarchSmem::bytes).  The radiation column blocks come after
@@ -102,9 +102,9 @@ __device__ __forceinline__ void march_block(const SubDev<T>& a, const int bid, d
   const int i00 = t0 * 32 + NGHOSTS, i10 = t1 * BY + NGHOSTS;
   const int N0 = a.N0, top = NGHOSTS + a.Nxx1, Nxx2 = a.Nxx2;
   const int nz = min(zc, Nxx2 - zf);
-  // substeps 2 and 4 sweep the planes the other way round: they start on the
-  // planes the substep before left in L2 (march_reversed)
-  const int z0 = NGHOSTS + (march_reversed(STAGE) ? Nxx2 - zf - nz : zf);
+  // a substep that sweeps the other way round starts on the planes that the
+  // substep before left in L2
+  const int z0 = NGHOSTS + (march_reversed<T, STAGE>(a) ? Nxx2 - zf - nz : zf);
   // element offsets fit in 32 bits (march_fits), so every address is one
   // 32-bit offset scaled onto a base pointer
   const unsigned N01 = (unsigned)a.N01, Ntot = (unsigned)a.Ntot;
@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(32 * BY, MINB)
   __shared__ bool last;
   pdl_enter();
   int lo = 0, hi = n - 1;
-  const int bx = march_reversed(STAGE) ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
+  const int bx = march_reversed<T, STAGE>(devs[0]) ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
     if (__ldg(offs + mid) <= bx)
@@ -477,6 +477,28 @@ void opt_in_shape() {
 }
 
 }  // namespace
+
+// When the launch's fields (11, in the correction form 13) are more than L2
+// holds: blocks run in index order, so sweeping every substep the same way
+// evicts each plane before the next substep comes to it.  Per RK4 step, one
+// direction -> alternating: 256x256x32 219 -> 212 us in FP64 and 151 -> 143.5 in
+// the correction form, four 192x192x24 grids in a batch 417 -> 401 us.  Where
+// the fields fit, alternating only puts a batch's radiation blocks last: one
+// 144x144x18 grid in the correction form 54.0 -> 58.0 us, 80x80x10 + 96x96x12 +
+// 144x144x18 in FP64 89.1 -> 90.9 (at the line, two 144x144x18 grids of 117 MB
+// 112.4 -> 113.6, three of 175 MB 164.7 -> 162.5).
+template <typename T>
+bool march_alternates(double points, bool corr) {
+  static int l2 = -1;
+  if (l2 < 0) {
+    int dev = 0;
+    NRPYELL_CUDA(cudaGetDevice(&dev));
+    NRPYELL_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev));
+  }
+  return points * (double)sizeof(T) * (corr ? 13 : 11) > (double)l2;
+}
+template bool march_alternates<double>(double, bool);
+template bool march_alternates<float>(double, bool);
 
 bool march_fits(const Dims& d) { return 3.0 * (double)d.Ntot < 4294967296.0; }
 

@@ -28,6 +28,7 @@ struct SubDev {
   int mbig, msmall;
   int n_tiles, n_col_blocks, ncol;
   int ncz;  // direct kernel: z-layers of its 3-D grid that hold the column blocks
+  int alternate;  // marching kernel: substeps 2 and 4 sweep from the last plane to the first (march_alternates)
   const T* __restrict__ S;     // stage input
   const T* y;                  // y_n (aliases out at stage 4)
   T* acc;
@@ -589,6 +590,12 @@ __device__ __forceinline__ int wrapm(int j, int Nxx2) {
 template <typename T>
 inline SubDev<T> make_dev(const SubstepArgs& a, int by, int p);
 
+// Whether the marching kernel's substeps sweep their planes (and, in a batch,
+// its grids) in turn upwards and downwards.  `points`: sum of the Ntot of a
+// launch's grids.
+template <typename T>
+bool march_alternates(double points, bool corr);
+
 // ---- batched launches (kernels_fused.cu, kernels_march.cu): the
 // shared-memory planes or marching kernel over many grids in one launch.
 // Launch arguments of one grid for the shape a.tile (kind 4 or 5).
@@ -624,6 +631,7 @@ inline SubDev<T> make_dev(const SubstepArgs& a, int by, int p) {
   f.mbig = f.tiles2;
   f.msmall = 0;
   f.ncz = 0;
+  f.alternate = march_alternates<T>((double)d.Ntot, a.R0 != nullptr);
   f.ncol = d.Nxx1 * d.Nxx2;
   f.S = (const T*)a.S;
   f.y = (const T*)a.y;

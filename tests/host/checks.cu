@@ -158,6 +158,10 @@ int check_stop_rule(double log10_tol, double volume, int check_every, const doub
   return g_faults;
 }
 
+int check_alternates(int fp64, double points) {
+  return fp64 ? march_alternates<double>(points, false) : march_alternates<float>(points, true);
+}
+
 // Jobs that end at the given steps of several launches.
 int check_start_state(const int* stop, int n) {
   g_faults = 0;

@@ -110,7 +110,9 @@ cudaError_t cudaLaunchCooperativeKernel(const void* f, dim3 g, dim3 b, void** a,
   return cudaSuccess;
 }
 cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
-  *v = a == cudaDevAttrMultiProcessorCount ? 148 : a == cudaDevAttrMaxSharedMemoryPerBlockOptin ? 232448 : 0;
+  *v = a == cudaDevAttrMultiProcessorCount ? 148
+     : a == cudaDevAttrMaxSharedMemoryPerBlockOptin ? 232448
+     : a == cudaDevAttrL2CacheSize ? 126 << 20 : 0;
   return cudaSuccess;
 }
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {

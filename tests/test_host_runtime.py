@@ -60,3 +60,13 @@ def test_training_order_is_not_reshuffled_under_its_copy(lib):
         want.append(list(perm))
     assert used == 4 * epochs * n
     np.testing.assert_array_equal(got[:epochs * n].reshape(epochs, n), want)
+
+
+@pytest.mark.parametrize("grids,fp64,alternates", [
+    ([(144, 144, 18)], 0, 0), ([(144, 144, 18)] * 3, 0, 0), ([(144, 144, 18)] * 5, 0, 1), ([(256, 256, 32)], 0, 1),
+    ([(144, 144, 18)] * 2, 1, 0), ([(144, 144, 18)] * 3, 1, 1), ([(192, 192, 24)], 1, 0), ([(224, 224, 28)], 1, 1)])
+def test_sweeps_alternate_beyond_l2_only(lib, grids, fp64, alternates):
+    """Where the fields of a launch fit in L2 (126 MiB here), sweeping back and
+    forth slows a batch by up to 8 %; beyond L2 it saves 3 to 6 %."""
+    points = sum((a + 10) * (b + 10) * (c + 10) for a, b, c in grids)
+    assert lib.check_alternates(fp64, C.c_double(points)) == alternates
