@@ -19,6 +19,70 @@
 
 namespace nrpyell {
 
+static bool same_dims(const Dims& a, const Dims& b) { return memcmp(&a, &b, sizeof(Dims)) == 0; }
+
+// A batch's routes.  On chip a team of equal grids runs alone, team after team,
+// at 1.6 (FP64) or 1.8 (FP32) times the cycles that its plan estimates, 1.9 GHz
+// (measured for 15 grids from 40x36x6 to 128x128x16 in teams of 1 to 16: 1.2 to
+// 2.0 and 1.2 to 2.2).  The batched launches run all other grids together: 28
+// (24) us a step, of which a batch saves nothing unless every grid leaves, and for each
+// grid 1.3 (1.1) us and its points at 9 G a second (14 G while the batch's fields
+// fit in L2, 12 G beyond; 1 to 16 grids of 48x48x6 to 144x144x18 took 0.83 to 1.13
+// times that in FP64, 0.9 to 1.5 in FP32).  So either all grids run on
+// chip, or those that take longer in the batch than on chip.  Microseconds per step,
+// on chip / in batched launches: FP64 48x48x6 + 64x64x8 + 80x80x10 38 / 45,
+// 16 x 112x112x14 328 / 394, 16 x 128x128x16 370 / 512; correction form 16 x 64x64x8
+// 69 / 91, 16 x 80x80x10 117 / 139, 16 x 128x128x16 356 / 371, 3 x 112x112x14 68 / 73,
+// 4 of them 92 / 87; 128x128x16 beside 112x112x14 and 144x144x18 92 / 88, two of each
+// 159 / 165.
+template <typename T>
+std::vector<int> chip_route(const std::vector<Dims>& grids) {
+  const bool fp64 = sizeof(T) == 8;
+  const int sms = sm_count();
+  const double us_per_cycle = (fp64 ? 1.6 : 1.8) / 1900.0;
+  struct Class {
+    Dims d;
+    std::vector<int> grids;
+    int team;
+    double chip, batch;  // us per RK4 step of all its grids
+  };
+  std::vector<Class> classes;
+  for (int c = 0; c < (int)grids.size(); c++) {
+    size_t k = 0;
+    while (k < classes.size() && !same_dims(classes[k].d, grids[c])) k++;
+    if (k == classes.size()) classes.push_back({grids[c], {}, 0, 0.0, 0.0});
+    classes[k].grids.push_back(c);
+  }
+  double total = 0.0;
+  for (const Dims& d : grids) total += (double)d.Ntot;
+  const double per_us = fp64 ? 9000.0 : march_alternates<T>(total, true) ? 12000.0 : 14000.0;
+  double chip = 0.0, batch = fp64 ? 28.0 : 24.0;
+  bool fit = true;
+  for (Class& k : classes) {
+    const int n = (int)k.grids.size();
+    const double points = (double)k.d.Nxx0 * k.d.Nxx1 * k.d.Nxx2;
+    k.team = resident_team<T>(k.d, n);
+    fit = fit && k.team > 0;
+    if (k.team > 0) {
+      const int rest = n % k.team;
+      k.chip = n / k.team * resident_plan<T>(k.d, sms / k.team).cost;
+      if (rest) k.chip += resident_plan<T>(k.d, sms / rest).cost;
+      k.chip *= 4.0 * us_per_cycle;
+    }
+    k.batch = n * ((fp64 ? 1.3 : 1.1) + points / per_us);
+    chip += k.chip;
+    batch += k.batch;
+  }
+  const bool all = fit && chip < batch;
+  std::vector<int> team(grids.size(), 0);
+  for (const Class& k : classes)
+    if (k.team > 0 && (all || k.chip < k.batch))
+      for (int c : k.grids) team[c] = k.team;
+  return team;
+}
+template std::vector<int> chip_route<double>(const std::vector<Dims>&);
+template std::vector<int> chip_route<float>(const std::vector<Dims>&);
+
 namespace {
 
 constexpr int kBatchStepsPerGraph = 16;
@@ -161,76 +225,34 @@ struct BatchResult {
   std::vector<double> last;
 };
 
-// Microseconds per RK4 step of one grid on chip, in teams of grids of its
-// dimensions (kernels_resident.cu); 0: it does not fit.  A substep takes
-// about 1.8 times the cycles that the plan estimates (measured from 64x64x8 to
-// 128x128x16), at 1.9 GHz.
-template <typename T>
-double resident_us(const Dims& d, int count, int* team) {
-  const ResTeam t = resident_team<T>(d, count);
-  *team = t.grids;
-  return t.grids ? 4.0 * t.cycles * 1.8 / 1900.0 : 0.0;
-}
-
-// Relaxes on chip the grids for which that is faster than their share of the
-// batched launches, team after team, and marks them in `done`.  Batched
-// launches run at about 6.5 G (FP64) and 10 G (FP32 correction form) points x
-// RK4 steps per second, but not below 26 us a step.  Measured per grid and
-// step at 128x128x16: 24 us on chip, 40 us in a batch (FP64).  256 steps of
-// twelve grids of 96x96x12, 128x128x16 and 192x192x24, all in batched launches ->
-// by this rule: 201 -> 171 ms; 512 steps of sixteen 128x128x16 grids in the
-// correction form: 213 -> 189 ms.
+// Relaxes on chip the grids that chip_route sends there, team after team, and
+// marks them in `done`.
 template <typename T>
 bool run_resident(const std::vector<Grid>& gs, std::vector<char>* done, BatchResult* out) {
   const int n = (int)gs.size();
-  const double points_per_us = sizeof(T) == 8 ? 6500.0 : 10000.0;
   done->assign(n, 0);
-  auto points = [](const Dims& d) { return (double)d.Nxx0 * d.Nxx1 * d.Nxx2; };
-  struct Class {
-    std::vector<int> grids;
-    int team;
-    double us;
-  };
-  std::vector<Class> classes;
-  double batch_us = 0.0, chip_us = 0.0;
-  bool all = true;
-  for (int c = 0; c < n; c++) {
-    const Dims& d = gs[c].d;
-    Class* k = nullptr;
-    for (Class& q : classes)
-      if (memcmp(&gs[q.grids[0]].d, &d, sizeof(Dims)) == 0) k = &q;
-    if (!k) {
-      classes.push_back(Class());
-      k = &classes.back();
+  std::vector<Dims> dims;
+  for (const Grid& G : gs) dims.push_back(G.d);
+  const std::vector<int> team = chip_route<T>(dims);
+  for (int first = 0; first < n; first++) {
+    if (team[first] == 0 || (*done)[first]) continue;
+    std::vector<int> members;
+    for (int c = first; c < n && (int)members.size() < team[first]; c++)
+      if (!(*done)[c] && same_dims(dims[c], dims[first])) members.push_back(c);
+    std::vector<ResGrid> grids;
+    for (int c : members) {
+      const Grid& G = gs[c];
+      grids.push_back({G.d, G.rt, G.bt, G.lt, G.b, G.rp, g_batch.state + kStateInts * c,
+                       g_batch.history + (size_t)c * g_batch.hist_len});
     }
-    k->grids.push_back(c);
-    batch_us += points(d) / points_per_us;
-  }
-  for (Class& k : classes) {
-    k.us = resident_us<T>(gs[k.grids[0]].d, (int)k.grids.size(), &k.team);
-    all = all && k.team > 0;
-    chip_us += k.us * k.grids.size();
-  }
-  all = all && chip_us < std::max(26.0, batch_us);
-  for (const Class& k : classes) {
-    if (k.team == 0 || !(all || k.us < points(gs[k.grids[0]].d) / points_per_us)) continue;
-    for (size_t at = 0; at < k.grids.size(); at += k.team) {
-      std::vector<ResGrid> team;
-      for (size_t i = at; i < std::min(k.grids.size(), at + k.team); i++) {
-        const int c = k.grids[i];
-        const Grid& G = gs[c];
-        team.push_back({G.d, G.rt, G.bt, G.lt, G.b, G.rp, g_batch.state + kStateInts * c,
-                        g_batch.history + (size_t)c * g_batch.hist_len});
-      }
-      std::vector<RelaxResult> r;
-      if (!relax_resident<T>(team, &r)) return false;
-      for (size_t i = 0; i < r.size(); i++) {
-        const int c = k.grids[at + i];
-        (*done)[c] = 1;
-        out->steps[c] = r[i].steps;
-        out->converged[c] = r[i].converged;
-        out->last[c] = r[i].last_log10_l2;
-      }
+    std::vector<RelaxResult> r;
+    if (!relax_resident<T>(grids, &r)) return false;
+    for (size_t i = 0; i < r.size(); i++) {
+      const int c = members[i];
+      (*done)[c] = 1;
+      out->steps[c] = r[i].steps;
+      out->converged[c] = r[i].converged;
+      out->last[c] = r[i].last_log10_l2;
     }
   }
   return true;

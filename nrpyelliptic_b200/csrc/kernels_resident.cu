@@ -1055,32 +1055,36 @@ template ResPlan resident_plan<float>(const Dims&, int);
 
 template <typename T>
 bool resident_ok(const Dims& d) {
-  return g_forced_tile < 0 && resident_plan<T>(d, device_attr(cudaDevAttrMultiProcessorCount)).blocks > 0;
+  return g_forced_tile < 0 && resident_plan<T>(d, sm_count()).blocks > 0;
 }
 template bool resident_ok<double>(const Dims&);
 template bool resident_ok<float>(const Dims&);
 
-// How many grids of these dimensions share the SMs best, and the estimated
-// cycles of a substep per grid (0 grids: they do not fit).  More grids at once
-// leave each fewer blocks, but their exchanges overlap.
+int sm_count() { return device_attr(cudaDevAttrMultiProcessorCount); }
+
+// More grids at once leave each fewer blocks, but their exchanges overlap.
 template <typename T>
-ResTeam resident_team(const Dims& d, int available) {
-  ResTeam best = {0, 0.0};
-  const int sms = device_attr(cudaDevAttrMultiProcessorCount);
+int resident_team(const Dims& d, int available) {
+  int best = 0;
+  double best_cost = 0.0;
+  const int sms = sm_count();
   for (int m = 1; m <= std::min(available, 16); m++) {
     const ResPlan p = resident_plan<T>(d, sms / m);
     if (p.blocks == 0) continue;
-    if (best.grids == 0 || p.cost / m < best.cycles) best = {m, p.cost / m};
+    if (best == 0 || p.cost / m < best_cost) {
+      best = m;
+      best_cost = p.cost / m;
+    }
   }
   return best;
 }
-template ResTeam resident_team<double>(const Dims&, int);
-template ResTeam resident_team<float>(const Dims&, int);
+template int resident_team<double>(const Dims&, int);
+template int resident_team<float>(const Dims&, int);
 
 template <typename T>
 bool relax_resident(const std::vector<ResGrid>& grids, std::vector<RelaxResult>* results) {
   const int n = (int)grids.size();
-  const int sms = device_attr(cudaDevAttrMultiProcessorCount);
+  const int sms = sm_count();
   std::vector<ResJob<T>> jobs(n);
   size_t slot_bytes = 0, share_bytes = 0;
   std::vector<size_t> slot_off(n), share_off(n);

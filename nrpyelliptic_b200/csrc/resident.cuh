@@ -86,12 +86,16 @@ ResPlan resident_plan(const Dims& d, int max_blocks);
 template <typename T>
 bool resident_ok(const Dims& d);
 
-struct ResTeam {
-  int grids;
-  double cycles;
-};
+// How many grids of these dimensions, of `available`, share the SMs best (0: they
+// do not fit).
 template <typename T>
-ResTeam resident_team(const Dims& d, int available);
+int resident_team(const Dims& d, int available);
+int sm_count();
+
+// Which grids of a batch relax on chip: the size of the teams for each grid, 0
+// for those that take the batched launches (batch.cu).
+template <typename T>
+std::vector<int> chip_route(const std::vector<Dims>& grids);
 
 // Relaxes the grids, all of the same dimensions, together in launches of many
 // RK4 steps; results[i] as relax_loop's.  Returns false on error.

@@ -4,6 +4,7 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <algorithm>
 #include <unordered_map>
 #include <vector>
 
@@ -156,6 +157,14 @@ int check_stop_rule(double log10_tol, double volume, int check_every, const doub
   g_fake_cooperative = nullptr;
   release_resident();
   return g_faults;
+}
+
+// Team sizes that a batch of n grids (Nxx, three ints each) gets, 0: batched launches.
+void route_of(int fp64, const int* nxx, int n, int* team) {
+  std::vector<Dims> d;
+  for (int i = 0; i < n; i++) d.push_back(FakeGrid(nxx[3 * i], nxx[3 * i + 1], nxx[3 * i + 2], -10.0, 0, 1.0).g.d);
+  const std::vector<int> t = fp64 ? chip_route<double>(d) : chip_route<float>(d);
+  std::copy(t.begin(), t.end(), team);
 }
 
 int check_alternates(int fp64, double points) {

@@ -70,3 +70,38 @@ def test_sweeps_alternate_beyond_l2_only(lib, grids, fp64, alternates):
     forth slows a batch by up to 8 %; beyond L2 it saves 3 to 6 %."""
     points = sum((a + 10) * (b + 10) * (c + 10) for a, b, c in grids)
     assert lib.check_alternates(fp64, C.c_double(points)) == alternates
+
+
+CUBE = {g: (g, g, n2) for g, n2 in ((48, 6), (64, 8), (80, 10), (96, 12), (112, 14), (128, 16), (144, 18))}
+
+
+@pytest.mark.parametrize("fp64,batch,chip", [
+    # microseconds per RK4 step on chip against batched launches
+    (1, [48, 64, 80], {48, 64, 80}),              # 38 / 45, and 54 with the smaller two in batched launches
+    (1, [48, 64, 80] * 4, {48, 64, 80}),          # 76 / 93
+    (1, [48, 48, 96] * 2, {48, 96}),              # 38 / 59
+    (0, [48, 48, 96] * 2, {48, 96}),              # 34 / 52
+    (0, [48, 48, 96] * 4, {48, 96}),              # 53 / 85
+    (1, [48] * 16, {48}),                         # 41 / 77
+    (0, [64] * 8, {64}),                          # 34 / 55
+    (0, [64] * 16, {64}),                         # 69 / 91
+    (0, [80] * 16, {80}),                         # 117 / 139
+    (1, [112] * 16, {112}),                       # 328 / 394
+    (1, [128] * 16, {128}),                       # 370 / 512
+    (0, [128] * 16, {128}),                       # 356 / 371
+    (0, [112] * 3, {112}),                        # 68 / 73
+    (0, [112] * 4, set()),                        # 92 / 87
+    (0, [112] * 8, set()),                        # 182 / 158
+    (0, [112] * 16, set()),                       # 361 / 298
+    (1, [64, 96, 144], set()),                    # a batch's fixed cost is paid in any case: 12 and 20 / 5 and 15
+    (0, [112, 128, 144], set()),                  # 92 with 128 on chip / 88
+    (0, [112, 128, 144] * 2, {128}),              # 159 / 165
+    (1, [128, 128, 144, 144], {128})])            # 23 / 30 each
+def test_batches_take_the_faster_route(lib, fp64, batch, chip):
+    """Routes of batches for which both were measured."""
+    nxx = np.array([CUBE[g] for g in batch], np.int32)
+    team = np.zeros(len(batch), np.int32)
+    ip = C.POINTER(C.c_int)
+    lib.route_of(fp64, nxx.ctypes.data_as(ip), len(batch), team.ctypes.data_as(ip))
+    assert {g for g, t in zip(batch, team) if t} == chip
+    assert all(t > 0 for g, t in zip(batch, team) if g in chip)
