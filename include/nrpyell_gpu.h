@@ -317,8 +317,12 @@ int nrpyell_relax_batch(int n, griddata_struct *grids, const REAL *dt, REAL log1
  * FP32 correction stretch of up to fold_every steps or to log10_switch, the
  * fold; FP64 steps from the switch on), and the stretches of all
  * configurations still in the FP32 phase, then their FP64 phases, run as
- * batches (on chip, or marching shapes for the FP32 stretches).  With the same
- * tile shapes each configuration's result is bitwise that of nrpyell_relax_mixed.
+ * batches (on chip, or marching shapes for the FP32 stretches).  Each
+ * configuration takes the steps of nrpyell_relax_mixed, bit for bit.  The norm of a
+ * residual is summed in an order that depends on the route and the tile shape, so
+ * final_log10_l2 agrees to rounding, and a run whose norm comes that close to a
+ * tolerance may stop a step earlier or later than alone; with a forced tile
+ * shape (nrpyell_set_tile) all results are bitwise those of nrpyell_relax_mixed.
  * steps_fp32[c], steps_fp64[c], final_log10_l2[c] as there (each array may
  * be NULL); the FP32 buffers (13 Ntot floats per configuration) stay
  * allocated for later calls until nrpyell_release_tables.  Returns the number

@@ -5,7 +5,8 @@ over several (one process per GPU, torchrun):
     python -m nrpyelliptic_b200.batch [--n 64] [--seed 20261203] [--tol -10] [--max-steps N] [--mixed]
     python -m torch.distributed.run --nproc-per-node 8 --master-addr 127.0.0.1 -m nrpyelliptic_b200.batch
 
-Every RK4 substep of all configurations -- on grids of different sizes -- is
+Configurations for which it is faster relax on chip, in teams of equal grids.
+Every RK4 substep of all others -- on grids of different sizes -- is
 one kernel launch; sixteen RK4 steps are one CUDA graph, replayed until every
 configuration has reached the tolerance (each stops on its own).  With
 --mixed the sweep runs the FP32 correction form (nrpyell_relax_batch_mixed,

@@ -54,7 +54,12 @@ namespace nrpyell {
 
 namespace {
 
-constexpr int kSlots = 8;            // substeps an exchanged value stays readable
+// Slots of an exchanged value, by substep.  A writer runs at most three substeps
+// ahead of a reader: neighbouring interior blocks, and a radiation block and the
+// face tiles of its rows, read each other; what else a radiation block reads (five
+// rows either side, seven columns of tiles at least five wide) lies at most two
+// tiles from one of those.
+constexpr int kSlots = 8;
 // Threads of a block: in an interior block 384 compute (three warpgroups) and
 // 128 fetch halos.  The launch's 128 registers per thread are divided 144 : 80.
 constexpr int kThreads = 512, kCompute = 384;
@@ -110,13 +115,15 @@ __device__ __forceinline__ void bar_arrive(int id, int n) {
 
 // ---------------------------------------------------------------- geometry
 
-// Columns x TX wide: a warp holds TX points along i0 times 32/TX rows.  The
-// row pitch of the shared uu tile (TX + 10 points) makes the rows of a warp
+// Row pitch of the shared uu tile (at least TX + 10 points): the rows of a warp
 // fall on different banks.
+constexpr int tile_pitch(bool fp64, int tx) { return fp64 ? (tx == 8 ? 24 : 26) : (tx == 8 ? 24 : 48); }
+
+// Columns x TX wide: a warp holds TX points along i0 times 32/TX rows.
 template <typename T, int TX>
 struct TileGeom {
   static constexpr int RPW = 32 / TX;
-  static constexpr int PITCH = sizeof(T) == 8 ? (TX == 8 ? 24 : 26) : (TX == 8 ? 24 : 48);
+  static constexpr int PITCH = tile_pitch(sizeof(T) == 8, TX);
 };
 
 __host__ __device__ constexpr int ceil_div(int a, int b) { return (a + b - 1) / b; }
@@ -907,9 +914,6 @@ int device_attr(cudaDeviceAttr a) {
   NRPYELL_CUDA(cudaDeviceGetAttribute(&v, a, dev));
   return v;
 }
-
-// Row pitch of the shared uu tile (TileGeom).
-int tile_pitch(bool fp64, int tx) { return fp64 ? (tx == 8 ? 24 : 26) : (tx == 8 ? 24 : 48); }
 
 constexpr int kTX[] = {8, 16};
 constexpr int kP[] = {1, 2, 3};  // planes of a thread per half

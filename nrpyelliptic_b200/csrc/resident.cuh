@@ -26,7 +26,7 @@ struct ResJob {
   const double* w;               // L2 weights
   // exchanged values tagged with the substep that wrote them (kernels_resident.cu):
   // uu on [i2][i1][xu_row >= Nxx0 + 5], vv on [i2][i1][12] (the last 7 planes along
-  // i0 and the outer 5), each in four rotating slots
+  // i0 and the outer 5), each in eight rotating slots
   void* xu;
   long long xu_slot;             // entries of a slot: uu, then vv from xv0 on
   int xu_row, xu_plane, xv0, xv_plane;

@@ -7,7 +7,8 @@ configuration's grid -- the table the autotuner chooses from.
 --mixed runs STEPS RK4 steps of the mixed-precision driver's FP32 correction
 form from the zero guess instead (after a warm-up of the same length) and
 prints the time per step: the launch to capture when profiling the FP32
-correction kernels.
+correction kernels.  Grids that fit on chip run there, without a tile shape,
+unless --tile forces one.
 
 For each shape: the stage-1, stage-2 and stage-4 kernels (CUDA-event time
 averaged over N launches replayed from a CUDA graph) and one whole RK4 step,
@@ -64,7 +65,8 @@ def sweep(name, launches=50, lib=None, only=None):
 
 def mixed_steps(name, steps, lib=None, tile=None):
     """Microseconds per RK4 step of the FP32 correction form (nrpyell_relax_mixed
-    with every step in FP32, folds every 256 steps) over `steps` steps."""
+    with every step in FP32, folds every 256 steps) over `steps` steps, the steps and
+    the tile shape (-1: on chip)."""
     import time
     lib = lib or _lib.load()
     prob = Problem(CONFIGS[name], lib=lib)
@@ -98,8 +100,8 @@ def main():
     if args.mixed:
         for name in args.configs:
             us, n, tile = mixed_steps(name, args.mixed, tile=args.tile)
-            print("%s: FP32 correction form, %d steps, %.2f us per RK4 step (wall clock, folds included), tile %d"
-                  % (name, n, us, tile))
+            print("%s: FP32 correction form, %d steps, %.2f us per RK4 step (wall clock, folds included), %s"
+                  % (name, n, us, "tile %d" % tile if tile >= 0 else "on chip"))
         return
     for name in args.configs:
         print("| %s | tile | 32 x by x planes | kind | stage 1 us | stage 2 us | stage 2 GB/s | stage 4 us | RK4 step us |"
