@@ -641,7 +641,7 @@ __device__ __forceinline__ void radiation_points(const double* f, const double* 
     const double* const f1 = f + 6 + jj;
 #pragma unroll
     for (int m = 0; m < 11; m++) u[m] = (m == 5) ? 0.0 : f1[(m - 5) * kRadPitch];
-    const double d1 = radiation_sum_x1(u);
+    const double d1 = radiation_sum_x1<true>(u);
     const double drf = radiation_drf(d0, d1, invdx0, invdx1, g[6 + jj], g[12 + jj]);
     const double fv = f1[0];
     if (jj < NGHOSTS) X[jj * n + q] = radiation_outgoing_neighbour(drf, fv, g[jj]);

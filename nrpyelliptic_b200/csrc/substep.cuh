@@ -14,8 +14,9 @@ namespace nrpyell {
 
 // Upwind first-derivative weights (one copy per translation unit).
 static __constant__ double c_fd1w[11][11] = NRPYELL_FD1_UPWIND_INIT;
-// The same as literals, where the index is known at compile time: constant
-// memory loads hoisted out of a time loop took 132 registers.
+// The same as literals, for the on-chip kernel, where constant memory loads hoisted
+// out of the time loop took 132 registers.  In the substep kernels literals are
+// slower (planes shape 32 x 8 x 1 at 160x150x20: 62.0 -> 62.4 us per RK4 step).
 static __device__ const double kFd1w[11][11] = NRPYELL_FD1_UPWIND_INIT;
 
 template <typename T>
@@ -296,11 +297,13 @@ __device__ __forceinline__ double radiation_sum_x0(const double* w, const double
   for (int m = 1; m < 11; m++) d = d + w[m] * v[m];
   return d;
 }
+template <bool LITERAL = false>
 __device__ __forceinline__ double radiation_sum_x1(const double* v) {
-  double d = kFd1w[5][0] * v[0];
+  const double* const w = LITERAL ? kFd1w[5] : c_fd1w[5];
+  double d = w[0] * v[0];
 #pragma unroll
   for (int m = 1; m < 11; m++)
-    if (m != 5) d = d + kFd1w[5][m] * v[m];
+    if (m != 5) d = d + w[m] * v[m];
   return d;
 }
 
@@ -315,8 +318,8 @@ __device__ __forceinline__ double radiation_drf(double d0, double d1, double inv
 // One outer layer of the radiation BC (apply_bcs_outerradiation_and_inner.c:
 // 400-407): the outgoing wave's d f/d r + f / r at the interior neighbour (X,
 // radius rn, cubed rn3) and at the point (Y, 1 / radius rinv), and the point's RHS from
-// the neighbour's, kprev.  The roundings are spelled out, so that the column
-// blocks and the on-chip radiation blocks agree bit for bit.
+// the neighbour's, kprev.  The roundings are spelled out, as in radiation_layers, so
+// that the on-chip radiation blocks and the column blocks agree bit for bit.
 __device__ __forceinline__ double radiation_outgoing_neighbour(double drf, double f, double rn) {
   return __dadd_rn(drf, __ddiv_rn(f, rn));
 }
@@ -334,14 +337,21 @@ __device__ __forceinline__ double radiation_layer(double cw, double kprev, doubl
 // the last interior point, drf/fvs the radial derivative and value at the
 // last interior point (index 0) and at layers 0..4 (1..5); colgeo the
 // column's radial geometry (r at index 0..5, stride N1).
+// radiation_layer's arithmetic, written so that the neighbour's term comes first in
+// every layer: with the terms of all layers up front (as the on-chip blocks have
+// them) the marching shapes took 1 to 2 % longer per RK4 step (32 x 8 x 4 at
+// 192x192x24 98.0 us instead of 96.8).
 __device__ __forceinline__ void radiation_layers(double cw, double kprev, const double* drf, const double* fvs,
                                                  const double* __restrict__ rcol, int N1, double* kk) {
 #pragma unroll
   for (int L = 0; L < NGHOSTS; L++) {
     const double rn = __ldg(rcol + L * N1);
-    const double rinv = 1.0 / __ldg(rcol + (L + 1) * N1);
-    kprev = radiation_layer(cw, kprev, radiation_outgoing_neighbour(drf[L], fvs[L], rn),
-                            radiation_outgoing_point(drf[L + 1], fvs[L + 1], rinv), radiation_r3(rn), rinv);
+    const double rr = __ldg(rcol + (L + 1) * N1);
+    const double X = drf[L] + fvs[L] / rn;
+    const double K = rn * rn * rn * __fma_rn(cw, X, kprev);
+    const double rinv = 1.0 / rr;
+    const double outw = -cw * __fma_rn(fvs[L + 1], rinv, drf[L + 1]);
+    kprev = __fma_rn(K * rinv * rinv, rinv, outw);
     kk[L] = kprev;
   }
 }
