@@ -272,7 +272,9 @@ bool run_batched_launches(const std::vector<Grid>& gs, bool corr, int* tile, Bat
   if (n == 0) return true;
   int max_steps = 0, max_tiles = 0;
   bool fits = true;
+  double points = 0.0;
   for (const Grid& G : gs) {
+    points += (double)G.d.Ntot;
     max_steps = std::max(max_steps, G.rp.max_steps);
     max_tiles = std::max(max_tiles, max_interior_blocks(G.d));
     fits = fits && march_fits(G.d);
@@ -282,6 +284,7 @@ bool run_batched_launches(const std::vector<Grid>& gs, bool corr, int* tile, Bat
     return false;
   }
   if (!ensure_batch(n, max_steps + 1, max_tiles)) return false;
+  const bool alternate = march_alternates<T>(points, corr);
   SubDev<T>* devs_dev = reinterpret_cast<SubDev<T>*>(g_batch.devs);
   std::vector<SubDev<T>> devs;
   std::vector<int> offs;
@@ -297,11 +300,11 @@ bool run_batched_launches(const std::vector<Grid>& gs, bool corr, int* tile, Bat
       if (!batch_tile_ok(t, corr) || (substep_tile_kind(t) == 5 && !fits)) continue;
       if (!build_devs<T>(gs, t, &devs, &offs, &blocks) || !upload_devs<T>(devs, offs)) return false;
       const SubDev<T>* d2 = devs_dev + 2 * n;  // stage 2: writes only k_even and the running total
-      launch_substep_batch<T>(2, false, t, d2, g_batch.offs, n, blocks, corr);
+      launch_substep_batch<T>(2, false, t, d2, g_batch.offs, n, blocks, corr, alternate);
       float tmin = 1e30f;
       for (int rep = 0; rep < 3; rep++) {
         NRPYELL_CUDA(cudaEventRecord(e0, stream()));
-        for (int i = 0; i < 5; i++) launch_substep_batch<T>(2, false, t, d2, g_batch.offs, n, blocks, corr);
+        for (int i = 0; i < 5; i++) launch_substep_batch<T>(2, false, t, d2, g_batch.offs, n, blocks, corr, alternate);
         NRPYELL_CUDA(cudaEventRecord(e1, stream()));
         NRPYELL_CUDA(cudaEventSynchronize(e1));
         float ms = 0;
@@ -327,9 +330,9 @@ bool run_batched_launches(const std::vector<Grid>& gs, bool corr, int* tile, Bat
   const long long launches_before = launch_count();
   NRPYELL_CUDA(cudaStreamBeginCapture(stream(), cudaStreamCaptureModeThreadLocal));
   for (int k = 0; k < kBatchStepsPerGraph; k++) {
-    launch_substep_batch<T>(1, true, *tile, devs_dev, g_batch.offs, n, blocks, corr);
+    launch_substep_batch<T>(1, true, *tile, devs_dev, g_batch.offs, n, blocks, corr, alternate);
     for (int st = 2; st <= 4; st++)
-      launch_substep_batch<T>(st, false, *tile, devs_dev + (size_t)st * n, g_batch.offs, n, blocks, corr);
+      launch_substep_batch<T>(st, false, *tile, devs_dev + (size_t)st * n, g_batch.offs, n, blocks, corr, alternate);
   }
   NRPYELL_CUDA(cudaStreamEndCapture(stream(), &graph));
   set_launch_count(launches_before);

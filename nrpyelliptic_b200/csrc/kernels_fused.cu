@@ -625,9 +625,9 @@ static void launch_batch_stage(int tile, const SubDev<T>* devs, const int* offs,
 
 template <typename T>
 void launch_substep_batch(int stage, bool resid, int tile, const SubDev<T>* devs, const int* offs, int n, int blocks,
-                          bool corr) {
+                          bool corr, bool alternate) {
   if (kTiles[tile].kind == 5) {  // batch_launch_dev checked march_fits for every grid
-    launch_march_batch<T>(stage, resid, kTiles[tile].v, devs, offs, n, blocks, corr);
+    launch_march_batch<T>(stage, resid, kTiles[tile].v, devs, offs, n, blocks, corr, alternate);
     return;
   }
   if (corr || sizeof(T) != 8) {
@@ -648,8 +648,8 @@ void launch_substep_batch(int stage, bool resid, int tile, const SubDev<T>* devs
     }
   }
 }
-template void launch_substep_batch<double>(int, bool, int, const SubDev<double>*, const int*, int, int, bool);
-template void launch_substep_batch<float>(int, bool, int, const SubDev<float>*, const int*, int, int, bool);
+template void launch_substep_batch<double>(int, bool, int, const SubDev<double>*, const int*, int, int, bool, bool);
+template void launch_substep_batch<float>(int, bool, int, const SubDev<float>*, const int*, int, int, bool, bool);
 
 template <typename T>
 void launch_ghost_fill(const Dims& d, const BcTables* bt, void* gfs) {

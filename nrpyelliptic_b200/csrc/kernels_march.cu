@@ -294,13 +294,14 @@ __global__ void __launch_bounds__(32 * BY, MINB) k_substep_march(SubDev<T> a) {
 // grid with its own launch arguments, stop test and done flag.
 template <typename T, int STAGE, bool RESID, int BY, int PZ, int D, int MINB, bool CORR = false>
 __global__ void __launch_bounds__(32 * BY, MINB)
-    k_substep_march_batch(const SubDev<T>* __restrict__ devs, const int* __restrict__ offs, int n) {
+    k_substep_march_batch(const SubDev<T>* __restrict__ devs, const int* __restrict__ offs, int n, bool alternate) {
   extern __shared__ __align__(16) double dsm[];
   __shared__ double sh[BY > 8 ? BY : 8];
   __shared__ bool last;
   pdl_enter();
   int lo = 0, hi = n - 1;
-  const int bx = march_reversed<T, STAGE>(devs[0]) ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
+  // a launch argument: read from devs[0] it would delay every block by a load
+  const int bx = (STAGE == 2 || STAGE == 4) && alternate ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
     if (__ldg(offs + mid) <= bx)
@@ -441,18 +442,18 @@ bool march_stage(int v, const SubstepArgs& a) {
 }
 
 template <typename T, int STAGE, bool RESID, int BY, int PZ, int D, int MINB, bool CORR = false>
-void launch_march_batch_shape(const SubDev<T>* devs, const int* offs, int n, int blocks) {
+void launch_march_batch_shape(const SubDev<T>* devs, const int* offs, int n, int blocks, bool alternate) {
   if (!march_opt_in<T, STAGE, RESID, BY, PZ, D, MINB, true, CORR>()) return;
   NRPYELL_LAUNCH_PDL((k_substep_march_batch<T, STAGE, RESID, BY, PZ, D, MINB, CORR>), blocks, 32 * BY,
-                     (MarchSmem<T, BY, STAGE, D, CORR>::bytes), devs, offs, n);
+                     (MarchSmem<T, BY, STAGE, D, CORR>::bytes), devs, offs, n, alternate);
 }
 
 template <typename T, int STAGE, bool RESID, bool CORR = false>
-bool march_batch_stage(int v, const SubDev<T>* devs, const int* offs, int n, int blocks) {
+bool march_batch_stage(int v, const SubDev<T>* devs, const int* offs, int n, int blocks, bool alternate) {
   switch (v) {
-#define NRPYELL_MARCH(I, BY, PZ, D, MINB)                                                 \
-  case I:                                                                                 \
-    launch_march_batch_shape<T, STAGE, RESID, BY, PZ, D, MINB, CORR>(devs, offs, n, blocks); \
+#define NRPYELL_MARCH(I, BY, PZ, D, MINB)                                                            \
+  case I:                                                                                            \
+    launch_march_batch_shape<T, STAGE, RESID, BY, PZ, D, MINB, CORR>(devs, offs, n, blocks, alternate); \
     return true;
     NRPYELL_MARCH_SHAPES(NRPYELL_MARCH)
 #undef NRPYELL_MARCH
@@ -561,18 +562,18 @@ template void prepare_march<float>(int);
 
 template <typename T>
 void launch_march_batch(int stage, bool resid, int v, const SubDev<T>* devs, const int* offs, int n, int blocks,
-                        bool corr) {
+                        bool corr, bool alternate) {
   bool ok = false;
   if (corr) {  // the correction form (FP32 only)
     if constexpr (sizeof(T) == 4) {
       switch (stage) {
         case 1:
-          ok = resid ? march_batch_stage<T, 1, true, true>(v, devs, offs, n, blocks)
-                     : march_batch_stage<T, 1, false, true>(v, devs, offs, n, blocks);
+          ok = resid ? march_batch_stage<T, 1, true, true>(v, devs, offs, n, blocks, alternate)
+                     : march_batch_stage<T, 1, false, true>(v, devs, offs, n, blocks, alternate);
           break;
-        case 2: ok = march_batch_stage<T, 2, false, true>(v, devs, offs, n, blocks); break;
-        case 3: ok = march_batch_stage<T, 3, false, true>(v, devs, offs, n, blocks); break;
-        default: ok = march_batch_stage<T, 4, false, true>(v, devs, offs, n, blocks); break;
+        case 2: ok = march_batch_stage<T, 2, false, true>(v, devs, offs, n, blocks, alternate); break;
+        case 3: ok = march_batch_stage<T, 3, false, true>(v, devs, offs, n, blocks, alternate); break;
+        default: ok = march_batch_stage<T, 4, false, true>(v, devs, offs, n, blocks, alternate); break;
       }
     }
     if (!ok) NRPYELL_FAIL("launch_march_batch: the correction form exists for FP32 only");
@@ -581,17 +582,17 @@ void launch_march_batch(int stage, bool resid, int v, const SubDev<T>* devs, con
   if constexpr (sizeof(T) == 8) {  // FP32 batches run the correction form only
     switch (stage) {
       case 1:
-        ok = resid ? march_batch_stage<T, 1, true>(v, devs, offs, n, blocks)
-                   : march_batch_stage<T, 1, false>(v, devs, offs, n, blocks);
+        ok = resid ? march_batch_stage<T, 1, true>(v, devs, offs, n, blocks, alternate)
+                   : march_batch_stage<T, 1, false>(v, devs, offs, n, blocks, alternate);
         break;
-      case 2: ok = march_batch_stage<T, 2, false>(v, devs, offs, n, blocks); break;
-      case 3: ok = march_batch_stage<T, 3, false>(v, devs, offs, n, blocks); break;
-      default: ok = march_batch_stage<T, 4, false>(v, devs, offs, n, blocks); break;
+      case 2: ok = march_batch_stage<T, 2, false>(v, devs, offs, n, blocks, alternate); break;
+      case 3: ok = march_batch_stage<T, 3, false>(v, devs, offs, n, blocks, alternate); break;
+      default: ok = march_batch_stage<T, 4, false>(v, devs, offs, n, blocks, alternate); break;
     }
   }
   if (!ok) NRPYELL_FAIL("launch_march_batch: no kernel for this shape and precision");
 }
-template void launch_march_batch<double>(int, bool, int, const SubDev<double>*, const int*, int, int, bool);
-template void launch_march_batch<float>(int, bool, int, const SubDev<float>*, const int*, int, int, bool);
+template void launch_march_batch<double>(int, bool, int, const SubDev<double>*, const int*, int, int, bool, bool);
+template void launch_march_batch<float>(int, bool, int, const SubDev<float>*, const int*, int, int, bool, bool);
 
 }  // namespace nrpyell
